@@ -132,7 +132,15 @@ typedef struct {
     int check_interval;            /* iterations per graph batch between host checks of the status word (4) */
     int restart_interval;          /* mixed: restart the Krylov recurrences at every n-th reliable update (1; 0: never) */
     int multigrid;                 /* mixed: 0: the reference preconditioner; 1: horizontal aggregation multigrid
-                                      V-cycle with the reference line relaxation as smoother on every level (0) */
+                                      V-cycle with the reference line relaxation as smoother on every level (0).
+                                      pcf_solve*, pcf_apply_corrector_device, pcf_implicit_step* and the ensemble
+                                      take the spectral preconditioner in its place (the inverse of the operator
+                                      averaged over each level: 4-10 iterations) while mg_dtau,
+                                      mg_coarse_iterations, mg_min_columns, mg_operator_bf16 and mg_smoother_fp8
+                                      are the defaults, no learned stage runs, nx, ny <= 4096 and nz <= 512; a
+                                      solve that has not converged after 24 such iterations goes on with the
+                                      V-cycle.  pcf_bicgstab always runs the V-cycle.  inner_tolerance counts
+                                      squared there: an update every second iteration instead of each */
     double mg_dtau;                /* multigrid: pseudo-time step of the smoother, all levels (2.5) */
     int mg_coarse_iterations;      /* multigrid: smoothing steps on the coarsest level (4) */
     int mg_min_columns;            /* multigrid: a level with at most this many columns is the coarsest (16) */
@@ -333,6 +341,14 @@ int pcf_multigrid_levels(pcf_handle *h, const pcf_params *prm, int cap, int *nle
 int pcf_multigrid_operator(pcf_handle *h, int level, double *coef);
 int pcf_apply_multigrid(pcf_handle *h, const double *sin, double *sout, const pcf_params *prm);
 
+/* The spectral preconditioner that solves with multigrid = 1 use in place of
+ * the V-cycle (see pcf_params.multigrid), applied once: sout = pi with
+ * (averaged operator) pi = sin in FP32 (host FP64 arrays, nx*ny*nz), for pi =
+ * s / fcscal.  The averaged operator has, on each level, the horizontal means
+ * of the difference form's six face couplings and of its defect.  PCF_ERANGE
+ * beyond nx, ny = 4096 or nz = 512 (such solves run the V-cycle). */
+int pcf_apply_spectral(pcf_handle *h, const double *sin, double *sout);
+
 /* Stencil tile autotuner (no reference counterpart).  One entry per device,
  * kernel family and grid size that a solve with pcf_params.autotune = 1 has
  * tuned: the chosen tile (tile_x threads along x, 128 threads per block, vec
@@ -407,7 +423,8 @@ enum pcf_prof_tag {
     PCF_PROF_PREDICT = 12,  /* implicit predictor with its predictand boundary fills (FP64) */
     PCF_PROF_CORRECT = 13,  /* corrector: dpip boundary fill and correct! (FP64) */
     PCF_PROF_MG_BF16 = 14,  /* V-cycle finest-level residual and smoothing stencils on the BF16 operator copy */
-    PCF_PROF_NTAGS = 15
+    PCF_PROF_SPECTRAL = 15, /* spectral preconditioner: transforms and column solves, FP32 */
+    PCF_PROF_NTAGS = 16
 };
 long long pcf_launch_count(const pcf_handle *h);
 /* Relative recursive residual after each BiCGSTAB iteration of the last

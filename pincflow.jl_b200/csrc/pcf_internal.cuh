@@ -153,6 +153,7 @@ struct ProfAcc {
 struct ProfState;   // defined in pcf_solver.cu
 struct GraphCache;  // captured iteration batches, defined in pcf_solver.cu
 struct MgState;     // multigrid hierarchy, defined in pcf_solver.cu
+struct SpectralState;  // spectral preconditioner, defined in pcf_solver.cu
 
 // ------------------------------------------------ shared memory, mbarriers --
 
@@ -246,6 +247,7 @@ struct pcf_handle {
     long long graph_launches;    // kernels in the graph being replayed
     pcf_net *net;                // learned warm start (not owned)
     pcf::MgState *mg;            // multigrid hierarchy (allocated on first use)
+    pcf::SpectralState *spec;    // spectral preconditioner (allocated on first use)
     float *lr32;                 // learned preconditioner stage: residual and correction (2 n, on first use)
     long long op_version;        // incremented whenever the operator changes
     // test hook (pcf_test_stall_staged_copy): 1 + the z-level whose staged

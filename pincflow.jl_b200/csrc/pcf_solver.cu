@@ -20,6 +20,7 @@
 
 #include "pcf_kernels.cuh"
 #include "pcf_mg.cuh"
+#include "pcf_spectral.cuh"
 #include "pcf_tiny.cuh"
 
 namespace {
@@ -1238,6 +1239,220 @@ static int mg_prepare(pcf_handle *h, const pcf_params *prm, bool ensemble = fals
     return PCF_OK;
 }
 
+// --------------------------------------------------- spectral preconditioner --
+// The inverse of the horizontally averaged operator (pcf_spectral.cuh) as the
+// right preconditioner of the FP32 loop, in place of the V-cycle.
+
+// Iterations a spectral solve gets to converge (4-10 on every grid tried); one
+// that has not by then goes on with the V-cycle from its last FP64 residual.
+constexpr int kSpectralIterations = 24;
+constexpr int kSpectralMaxLevels = 512;  // column solves: 32 runs of at most 16 levels
+
+struct SpectralState {
+    SpectralArgs a{};
+    dim3 gx, gy, gz, bz;
+    size_t smx = 0, smy = 0;  // dynamic shared memory of the x and y transforms
+    int ch = 0;               // levels per run of the column solves
+    double *part = nullptr, *lev = nullptr;
+    float *lad = nullptr, *piv = nullptr;
+    long long version = -1;   // operator version of the pivots
+    std::vector<void *> allocs;
+};
+
+// Whether a solve may replace the V-cycle by the spectral preconditioner: the
+// V-cycle's own settings are the defaults (others ask for that V-cycle), no
+// learned stage (trained on the V-cycle), and extents the kernels take.
+static bool spectral_applies(const pcf_handle *h, const pcf_params *prm) {
+    pcf_params def;
+    pcf_params_default(&def);
+    return prm->multigrid && prm->precision == PCF_PRECISION_MIXED && prm->preconditioner &&
+           prm->mg_dtau == def.mg_dtau && prm->mg_coarse_iterations == def.mg_coarse_iterations &&
+           prm->mg_min_columns == def.mg_min_columns && prm->mg_operator_bf16 == def.mg_operator_bf16 &&
+           prm->mg_smoother_fp8 == def.mg_smoother_fp8 && !((prm->learned & 2) && h->net) && !h->test_stall &&
+           h->d.nx <= kFftMaxLength && h->d.ny <= kFftMaxLength && h->d.nz <= kSpectralMaxLevels;
+}
+
+static void spectral_free(pcf_handle *h) {
+    if (!h->spec) return;
+    for (void *q : h->spec->allocs) cudaFree(q);
+    delete h->spec;
+    h->spec = nullptr;
+}
+
+static void fft_plan(FftPlan *p, int n) {
+    p->n = n;
+    p->nst = 0;
+    int rest = n, ns = 1;
+    auto add = [&](int r) {
+        p->radix[p->nst] = r;
+        p->m[p->nst].set((unsigned)(n / r));
+        p->ns[p->nst].set((unsigned)ns);
+        ++p->nst;
+        ns *= r;
+        rest /= r;
+    };
+    while (rest % 8 == 0 && rest != 16) add(8);  // 16 as 4 x 4
+    for (int r : {4, 2, 3, 5, 7})
+        while (rest % r == 0) add(r);
+    for (int r = 11; rest > 1; r += 2)
+        while (rest % r == 0) add(r);
+}
+
+// Buffers, transform plans and launch shapes (first call on the handle).
+static int spectral_create(pcf_handle *h) {
+    SpectralState *s = new SpectralState();
+    h->spec = s;
+    auto alloc = [&](void **q, size_t bytes) -> int {
+        const cudaError_t e = cudaMalloc(q, bytes);
+        if (e != cudaSuccess) return pcf_set_cuda_error(e);
+        s->allocs.push_back(*q);
+        h->bytes += (long long)bytes;
+        return PCF_OK;
+    };
+    SpectralArgs &a = s->a;
+    const int nx = h->d.nx, ny = h->d.ny, nz = h->d.nz;
+    a.nx = nx;
+    a.ny = ny;
+    a.nz = nz;
+    a.npair = (nx + 1) / 2;
+    a.nxs = (2 * a.npair + 7) / 8 * 8;  // rows start on a 32-byte sector
+    a.rows = (long long)ny * nz;
+    a.n = h->d.n;
+    a.nspec = a.rows * a.nxs;
+    a.nkx = nx / 2 + 1;
+    a.nky = ny / 2 + 1;
+    a.scale = (float)(1.0 / ((double)nx * ny));
+    a.dper.set((unsigned)(nx % 4 == 0 ? nx / 4 : nx));
+    a.dpair.set((unsigned)a.npair);
+    int rc;
+    float2 *tw = nullptr;
+    if ((rc = alloc((void **)&a.spec, sizeof(float) * (size_t)a.nspec)) ||
+        (rc = alloc((void **)&s->piv, sizeof(float) * (size_t)nz * a.nkx * a.nky)) ||
+        (rc = alloc((void **)&s->part, sizeof(double) * (size_t)nz * kLevelBlocks * kLevelSums)) ||
+        (rc = alloc((void **)&s->lev, sizeof(double) * (size_t)nz * kLevelSums)) ||
+        (rc = alloc((void **)&s->lad, sizeof(float) * 2 * (size_t)nz)) ||
+        (rc = alloc((void **)&tw, sizeof(float2) * (size_t)(nx + ny)))) {
+        spectral_free(h);
+        return rc;
+    }
+    a.piv = s->piv;
+    a.lad = s->lad;
+    a.lau = s->lad + nz;
+    fft_plan(&a.fx, nx);
+    fft_plan(&a.fy, ny);
+    std::vector<float2> host((size_t)(nx + ny));
+    for (int q = 0; q < nx + ny; ++q) {
+        const double t = -2.0 * 3.14159265358979323846 * (q < nx ? (double)q / nx : (double)(q - nx) / ny);
+        host[q] = make_float2((float)std::cos(t), (float)std::sin(t));
+    }
+    a.fx.tw = tw;
+    a.fy.tw = tw + nx;
+    cudaError_t e = cudaMemcpy(tw, host.data(), sizeof(float2) * host.size(), cudaMemcpyHostToDevice);
+    // x: row pairs per block, y: pairs per block; about 2048 values in flight a
+    // block, fewer where that leaves less than two blocks per SM
+    const long long pairs = (a.rows + 1) / 2;
+    const long long want = 2LL * num_sms();
+    int lx = (int)std::max<long long>(1, std::min<long long>(2048 / nx, pairs / want));
+    int ly = std::max(4, 2048 / ny);
+    while (ly > 4 && (long long)((a.npair + ly - 1) / ly) * nz < want) ly /= 2;
+    ly = std::min(ly, std::max(1, 8192 / ny));
+    s->gx = dim3((unsigned)((pairs + lx - 1) / lx));
+    s->gy = dim3((unsigned)((a.npair + ly - 1) / ly), (unsigned)nz);
+    s->smx = 2 * sizeof(float2) * (size_t)fpad_size(lx * nx);
+    s->smy = 2 * sizeof(float2) * (size_t)fpad_size(ly * ny);
+    s->ch = nz <= 128 ? 4 : nz <= 256 ? 8 : 16;
+    s->gz = dim3((unsigned)((a.npair + 31) / 32), (unsigned)ny);
+    s->bz = dim3(32, (unsigned)((nz + s->ch - 1) / s->ch));
+    a.lines = lx;  // the y kernels' count is set at their launches
+    a.dl.set((unsigned)lx);
+    // the kernels' shared-memory limit, raised before any launch that may be captured
+    const int limit = 2 * (int)sizeof(float2) * fpad_size(8192);
+    const void *kernels[] = {(const void *)k_spec_x<TH_B, true>,    (const void *)k_spec_x<TH_B, false>,
+                             (const void *)k_spec_x<TH_PUPD, true>, (const void *)k_spec_x<TH_PUPD, false>,
+                             (const void *)k_spec_x<TH_SUPD, true>, (const void *)k_spec_x<TH_SUPD, false>,
+                             (const void *)k_spec_xinv<true>,       (const void *)k_spec_xinv<false>,
+                             (const void *)k_spec_y<false>,         (const void *)k_spec_y<true>};
+    for (const void *k : kernels)
+        if (e == cudaSuccess) e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, limit);
+    if (e != cudaSuccess) {
+        spectral_free(h);
+        return pcf_set_cuda_error(e);
+    }
+    return PCF_OK;
+}
+
+// Level means and pivots of the current operator.
+static int spectral_prepare(pcf_handle *h) {
+    int rc;
+    if (!h->spec && (rc = spectral_create(h))) return rc;
+    SpectralState &s = *h->spec;
+    if (s.version == h->op_version) return PCF_OK;
+    const SpectralArgs &a = s.a;
+    ProfScope ps(h, PCF_PROF_ASSEMBLE, 7.0 * 4 * (double)h->d.n + 4.0 * a.nz * a.nkx * a.nky, 3);
+    const int nblk = std::max(1, std::min(kLevelBlocks, std::min((h->d.plane + 255) / 256, 16 * num_sms() / a.nz + 1)));
+    k_level_sums<<<dim3((unsigned)nblk, (unsigned)a.nz), 256, 0, h->stream>>>(h->coefB32, h->d.plane, h->d.n, s.part);
+    k_level_means<<<(unsigned)((kLevelSums * a.nz + 127) / 128), 128, 0, h->stream>>>(s.part, nblk, h->d.plane, a.nz,
+                                                                                       s.lev, s.lad, s.lad + a.nz);
+    k_spec_pivots<<<(unsigned)((a.nkx * a.nky + 127) / 128), 128, 0, h->stream>>>(s.lev, a.nx, a.ny, a.nz, a.nkx,
+                                                                                   a.nky, s.piv);
+    PCF_CUDA_TRY(cudaGetLastError());
+    s.version = h->op_version;
+    return PCF_OK;
+}
+
+// out = (averaged operator)^-1 of the vector formed by MODE (bvec itself, or
+// the BiCGSTAB p / s update written back to bvec), in pi = s / fcscal.
+template <int MODE>
+static int spectral_precond(pcf_handle *h, const Work<float> &w, float *bvec, float *out,
+                            const KrylovScalars *guard) {
+    SpectralState &s = *h->spec;
+    SpectralArgs a = s.a;
+    a.in = bvec;
+    a.r = w.r;
+    a.v = w.v;
+    a.vec = bvec;
+    a.out = out;
+    a.scal = guard;
+    const bool vec = a.nx % 4 == 0;
+    const double sb = 4.0 * (double)a.nspec, nb = 4.0 * (double)a.n;
+    SpectralArgs y = a;
+    y.lines = (int)((a.npair + s.gy.x - 1) / s.gy.x);
+    y.dl.set((unsigned)y.lines);
+    {
+        ProfScope ps(h, PCF_PROF_SPECTRAL, sb + (MODE == TH_B ? 1 : MODE == TH_PUPD ? 4 : 3) * nb);
+        if (vec)
+            k_spec_x<MODE, true><<<s.gx, kFftThreads, s.smx, h->stream>>>(a);
+        else
+            k_spec_x<MODE, false><<<s.gx, kFftThreads, s.smx, h->stream>>>(a);
+    }
+    if (a.ny > 1) {
+        ProfScope ps(h, PCF_PROF_SPECTRAL, 2 * sb);
+        k_spec_y<false><<<s.gy, kFftThreads, s.smy, h->stream>>>(y);
+    }
+    {
+        ProfScope ps(h, PCF_PROF_SPECTRAL, 2 * sb + nb / 4);
+        if (s.ch == 4)
+            k_spec_z<4><<<s.gz, s.bz, 0, h->stream>>>(a);
+        else if (s.ch == 8)
+            k_spec_z<8><<<s.gz, s.bz, 0, h->stream>>>(a);
+        else
+            k_spec_z<16><<<s.gz, s.bz, 0, h->stream>>>(a);
+    }
+    if (a.ny > 1) {
+        ProfScope ps(h, PCF_PROF_SPECTRAL, 2 * sb);
+        k_spec_y<true><<<s.gy, kFftThreads, s.smy, h->stream>>>(y);
+    }
+    {
+        ProfScope ps(h, PCF_PROF_SPECTRAL, sb + nb);
+        if (vec)
+            k_spec_xinv<true><<<s.gx, kFftThreads, s.smx, h->stream>>>(a);
+        else
+            k_spec_xinv<false><<<s.gx, kFftThreads, s.smx, h->stream>>>(a);
+    }
+    PCF_CUDA_TRY(cudaGetLastError());
+    return PCF_OK;
+}
+
 // Tunes the stencil families that a solve with these settings launches
 // (before its iteration batches are captured).
 static int autotune_handle(pcf_handle *h, const pcf_params *prm) {
@@ -1269,6 +1484,7 @@ struct LoopCfg {
     int flex;      // accumulate x from the preconditioned directions (FP32 inner loop)
     int reliable;  // fold into the FP64 solution and restart r from the true residual
     int mg = 0;    // multigrid V-cycle as the preconditioner (FP32 loop only)
+    int sp = 0;    // spectral preconditioner (FP32 loop only)
     int learned_pc = 0;  // learned stage after the preconditioner (FP32 loop only)
 };
 
@@ -1339,7 +1555,9 @@ static int bicgstab_iteration(pcf_handle *h, const Work<T> &w, const LoopCfg &c)
     if (c.precond) {
         if constexpr (sizeof(T) == 4) {
             const float *post = c.learned_pc ? nullptr : w.post;
-            if (c.mg)
+            if (c.sp)
+                rc = spectral_precond<TH_PUPD>(h, w, w.p, z = w.za, w.scal);
+            else if (c.mg)
                 rc = mg_precond<TH_PUPD>(h, w, w.p, w.scal, &z, w.za, w.zb, post);
             else
                 rc = precond_apply<T, TH_PUPD>(h, w, w.p, c.pc_iters, c.deta, w.scal, &z, nullptr, nullptr, post);
@@ -1375,7 +1593,10 @@ static int bicgstab_iteration(pcf_handle *h, const Work<T> &w, const LoopCfg &c)
         const T *post = w.post;
         if constexpr (sizeof(T) == 4) {
             if (c.learned_pc) post = nullptr;
-            if (c.mg) {
+            if (c.sp) {
+                rc = spectral_precond<TH_SUPD>(h, w, w.s, z = w.zc, w.scal);
+                done = true;
+            } else if (c.mg) {
                 rc = mg_precond<TH_SUPD>(h, w, w.s, w.scal, &z, w.zc, w.zd, post);
                 done = true;
             }
@@ -1450,12 +1671,13 @@ struct GraphKey {
     int tsize, precond, pc_iters, flex, reliable, pi, batch;
     double deta;
     int mg, mg_levels, mg_coarse_iters, mg_bf16;
+    int sp;           // spectral preconditioner
     const void *net;  // the learned stage's network (null: no stage)
     bool operator==(const GraphKey &o) const {
         return tsize == o.tsize && precond == o.precond && pc_iters == o.pc_iters && flex == o.flex &&
                reliable == o.reliable && pi == o.pi && batch == o.batch && deta == o.deta && mg == o.mg &&
                mg_levels == o.mg_levels && mg_coarse_iters == o.mg_coarse_iters && mg_bf16 == o.mg_bf16 &&
-               net == o.net;
+               sp == o.sp && net == o.net;
     }
 };
 struct GraphEntry {
@@ -1574,7 +1796,7 @@ static GraphKey graph_key(const pcf_handle *h, int tsize, const LoopCfg &c, bool
     return GraphKey{tsize, c.precond, c.pc_iters, c.flex, c.reliable, pi, check_interval, c.deta, c.mg,
                     c.mg && h->mg ? (int)h->mg->lv.size() : 0, c.mg && h->mg ? h->mg->coarse_iters : 0,
                     c.mg && h->mg ? (int)h->mg->bf16 | (h->mg->lv[0].tmap8 ? 2 : 0) | (h->mg->fused_from + 1) << 2 : 0,
-                    c.learned_pc ? (const void *)h->net : nullptr};
+                    c.sp, c.learned_pc ? (const void *)h->net : nullptr};
 }
 
 // A complete BiCGSTAB run: run_start, the iteration batches, run_finish.
@@ -1757,6 +1979,7 @@ int pcf_destroy(pcf_handle *h) {
         mg_free(h);
         delete h->mg;
     }
+    spectral_free(h);
     if (h->prof) {
         for (cudaEvent_t e : h->prof->pool) cudaEventDestroy(e);
         delete h->prof;
@@ -2101,6 +2324,23 @@ int pcf_apply_multigrid(pcf_handle *h, const double *sin_, double *sout, const p
     rc = mg_precond<TH_B>(h, work32(h), h->s32, nullptr, &z, h->za32, h->zb32, nullptr);
     if (rc) return rc;
     k_to_double<<<vec_grid(h->d.n), 256, 0, h->stream>>>(z, h->w64, h->d.n);
+    PCF_CUDA_TRY(cudaGetLastError());
+    PCF_CUDA_TRY(cudaMemcpyAsync(sout, h->w64, sizeof(double) * h->d.n, cudaMemcpyDeviceToHost, h->stream));
+    PCF_CUDA_TRY(cudaStreamSynchronize(h->stream));
+    return PCF_OK;
+}
+
+int pcf_apply_spectral(pcf_handle *h, const double *sin_, double *sout) {
+    if (!h || !sin_ || !sout) return PCF_EINVAL;
+    if (!h->operator_set) return PCF_ENOTREADY;
+    if (h->d.nx > kFftMaxLength || h->d.ny > kFftMaxLength || h->d.nz > kSpectralMaxLevels) return PCF_ERANGE;
+    PCF_CUDA_TRY(cudaSetDevice(h->dims.device));
+    int rc = spectral_prepare(h);
+    if (rc) return rc;
+    if ((rc = upload_vec(h, sin_, h->b64, h->s32))) return rc;
+    if ((rc = spectral_precond<TH_B>(h, work32(h), h->s32, h->za32, nullptr))) return rc;
+    k_to_double<<<vec_grid(h->d.n), 256, 0, h->stream>>>(h->za32, h->w64, h->d.n);
+    h->launches += 1;
     PCF_CUDA_TRY(cudaGetLastError());
     PCF_CUDA_TRY(cudaMemcpyAsync(sout, h->w64, sizeof(double) * h->d.n, cudaMemcpyDeviceToHost, h->stream));
     PCF_CUDA_TRY(cudaStreamSynchronize(h->stream));
@@ -2559,9 +2799,27 @@ static int tiny_solve(pcf_handle *h, double tol, const pcf_params *prm, const do
 // the benchmark grids) is dropped like one that breaks down.
 constexpr int kStageIterations = 60;
 
+// Residual drop that triggers a reliable update.  A spectral iteration alone
+// falls by more than inner_tolerance, so its updates come at the square (every
+// second iteration); an update per iteration would cost an FP64 apply and a
+// Krylov restart each.
+static double ru_delta(const pcf_params *prm, const LoopCfg &c) {
+    return c.sp ? prm->inner_tolerance * prm->inner_tolerance : prm->inner_tolerance;
+}
+
+// Tolerance of the iteration.  What a spectral iteration leaves of the residual
+// lies over the terrain (its largest value 40 to 200 times its RMS, the
+// V-cycle's about 10), so it is asked for a tenth of the caller's tolerance:
+// the winds corrected with the pressure are then as close to the exact ones
+// there as after a V-cycle solve (w over a 1 km mountain, tolerance 1e-10: 1e-6
+// of its RMS instead of 4e-5).  Most solves end below that anyway.
+static double loop_tolerance(double tol, const LoopCfg &c) { return c.sp ? 0.1 * tol : tol; }
+
 // Solves A x = b64 (device) according to prm; the solution ends in *xres
 // (a device FP64 buffer owned by the handle).
-static int krylov_solve(pcf_handle *h, double tolref, const pcf_params *prm, const double **xres, pcf_result *res) {
+// spectral: the caller lets the spectral preconditioner stand in for the V-cycle (spectral_applies).
+static int krylov_solve(pcf_handle *h, double tolref, const pcf_params *prm, const double **xres, pcf_result *res,
+                        bool spectral = false) {
     const double tol = prm->tolerance_is_relative ? prm->tolerance : prm->tolerance / tolref;  // :49-53
     LoopCfg c;
     c.precond = prm->preconditioner;
@@ -2637,10 +2895,20 @@ static int krylov_solve(pcf_handle *h, double tolref, const pcf_params *prm, con
     LoopCfg cm = c;
     cm.flex = 1;
     cm.reliable = 1;
-    if (prm->multigrid) {
-        if ((rc = mg_prepare(h, prm))) return rc;
+    auto use_vcycle = [&]() -> int {
+        cm.sp = 0;
+        const int r = mg_prepare(h, prm);
+        if (r) return r;
         cm.mg = 1;
         cm.deta = h->mg->lv[0].deta;
+        return PCF_OK;
+    };
+    if (spectral && spectral_applies(h, prm)) {
+        if ((rc = spectral_prepare(h))) return rc;
+        cm.sp = 1;
+        cm.deta = 0;
+    } else if (prm->multigrid && (rc = use_vcycle())) {
+        return rc;
     }
     if (prm->autotune && (rc = autotune_handle(h, prm))) return rc;
     if ((prm->learned & 2) && h->net && c.precond) {
@@ -2661,23 +2929,31 @@ static int krylov_solve(pcf_handle *h, double tolref, const pcf_params *prm, con
         float *e = nullptr;
         RunOut ro;
         // with the learned stage the iteration gets kStageIterations to converge
-        const int cap = cm.learned_pc ? std::min(maxit - res->niter, kStageIterations) : maxit - res->niter;
-        rc = bicgstab_run<float>(h, w, w.s, tol, cap, cm, prm->check_interval, false, &e, &ro, res->niter, 1.0,
-                                 b_norm, prm->inner_tolerance, prm->restart_interval);
+        // and likewise with the spectral preconditioner
+        const int cap = std::min(maxit - res->niter, cm.learned_pc ? kStageIterations
+                                                     : cm.sp       ? kSpectralIterations
+                                                                   : maxit);
+        rc = bicgstab_run<float>(h, w, w.s, loop_tolerance(tol, cm), cap, cm, prm->check_interval, false, &e, &ro, res->niter, 1.0,
+                                 b_norm, ru_delta(prm, cm), prm->restart_interval);
         if (rc) return rc;
         res->niter += ro.iters;
         res->nrefine += ro.nupdates;
         reliable_bytes(h, ro.nupdates);
         if (ro.nupdates > 0) rel = ro.res;
-        if (ro.converged) break;
-        const bool stalled = cm.learned_pc && ro.iters >= cap && res->niter < maxit;
-        if ((ro.status == PCF_EBREAKDOWN || stalled) && restarts < prm->max_refinements && res->niter < maxit) {
+        if (ro.converged || (cm.sp && ro.status == PCF_OK && rel <= tol)) break;
+        const bool stalled = (cm.learned_pc || cm.sp) && ro.iters >= cap && res->niter < maxit;
+        if ((ro.status == PCF_EBREAKDOWN || stalled) && (cm.sp || restarts < prm->max_refinements) &&
+            res->niter < maxit) {
+            restarts += cm.sp ? 0 : 1;  // leaving the spectral preconditioner is not one of them
             if (cm.learned_pc) {
                 // the plain preconditioner is the fallback: a breakdown, divergence or
                 // stall with the learned stage drops the stage for the rest of the solve
                 // and discards the FP32 correction since the last reliable update
                 // (the FP64 solution keeps every reliable update made with it)
                 cm.learned_pc = 0;
+            } else if (cm.sp) {
+                // likewise the V-cycle for the spectral preconditioner
+                if ((rc = use_vcycle())) return rc;
             } else {
                 // fold what the broken-down iteration accumulated
                 k_axpy_f2d<<<vec_grid(h->d.n), 256, 0, h->stream>>>(w.x, h->x64, h->fc64, h->d.n, b_norm);
@@ -2687,7 +2963,6 @@ static int krylov_solve(pcf_handle *h, double tolref, const pcf_params *prm, con
             // restart from the true residual
             if ((rc = true_residual(h, h->b64, h->x64, &rnorm))) return rc;
             rel = rnorm / b_norm;
-            restarts += 1;
             if (!std::isfinite(rel)) {
                 res->status = PCF_ENONFINITE;
                 break;
@@ -2730,7 +3005,7 @@ static int solve_common(pcf_handle *h, double dt, double rf, double tolref, cons
     PCF_CUDA_TRY(cudaEventRecord(h->ev[2], h->stream));
     {
         NvtxScope r("pcf krylov");
-        if ((rc = krylov_solve(h, tolref, prm, x, res))) return rc;
+        if ((rc = krylov_solve(h, tolref, prm, x, res, true))) return rc;
     }
     PCF_CUDA_TRY(cudaEventRecord(h->ev[3], h->stream));
     return PCF_OK;
@@ -2963,6 +3238,7 @@ struct pcf_ensemble {
     long long graph_launches = 0;
     long long launches = 0;
     bool key_valid = false;
+    bool use_sp = false, key_sp = false;  // spectral preconditioner: this solve's, the captured graph's
     int key_ci = 0, key_precond = 0, key_pc_iters = 0, key_mg = 0, key_mg_ci = 0, key_mg_min = 0, key_maxit = 0;
     double key_dtau = 0, key_mg_dtau = 0;
     KrylovScalars *h_status = nullptr;  // pinned, 2 slots x members
@@ -2987,14 +3263,15 @@ __global__ void k_ensemble_continue(KrylovScalars *const *scal, int n, int *batc
     cudaGraphSetConditional(cond, (any && b < max_batches) ? 1u : 0u);
 }
 
-static LoopCfg ensemble_loop_cfg(pcf_handle *h, const pcf_params *prm) {
+static LoopCfg ensemble_loop_cfg(const pcf_ensemble *e, pcf_handle *h, const pcf_params *prm) {
     LoopCfg c;
     c.precond = prm->preconditioner;
     c.pc_iters = prm->preconditioner_iterations;
     c.deta = deta_of(h, prm->dtau);
     c.flex = 1;
     c.reliable = 1;
-    c.mg = prm->multigrid ? 1 : 0;
+    c.sp = e->use_sp ? 1 : 0;
+    c.mg = prm->multigrid && !c.sp ? 1 : 0;
     if (c.mg) c.deta = h->mg->lv[0].deta;
     return c;
 }
@@ -3011,7 +3288,7 @@ static int ensemble_record_batch(pcf_ensemble *e, const pcf_params *prm, int ci,
         pcf_handle *h = e->m[q];
         ce = cudaStreamWaitEvent(h->stream, e->fork, 0);
         if (ce != cudaSuccess) break;
-        const LoopCfg c = ensemble_loop_cfg(h, prm);
+        const LoopCfg c = ensemble_loop_cfg(e, h, prm);
         const Work<float> w = work32_pi(h);
         for (int it = 0; it < ci && rc == PCF_OK; ++it) rc = bicgstab_iteration<float>(h, w, c);
         if (rc) break;
@@ -3119,6 +3396,7 @@ static int ensemble_capture(pcf_ensemble *e, const pcf_params *prm, int ci) {
     e->key_mg_min = prm->mg_min_columns;
     e->key_mg_dtau = prm->mg_dtau;
     e->key_maxit = prm->poisson_iterations;
+    e->key_sp = e->use_sp;
     return ensemble_capture_loop(e, prm, ci, (prm->poisson_iterations + ci - 1) / ci);
 }
 
@@ -3193,6 +3471,9 @@ int pcf_ensemble_solve_device(pcf_ensemble *e, const double *const *d_rhs, const
     const int ci = prm->check_interval < 1 ? 16 : prm->check_interval;
     const int maxit = prm->poisson_iterations;
     int rc;
+    e->use_sp = true;
+    for (int q = 0; q < n; ++q) e->use_sp = e->use_sp && spectral_applies(e->m[q], prm);
+    const int cap = e->use_sp ? std::min(maxit, kSpectralIterations) : maxit;
     PCF_CUDA_TRY(cudaEventRecord(e->t0, e->origin));
     // setup on every member's stream: inputs, assembly, pivots, multigrid
     // hierarchy, r = b - A 0 in FP64 with its norm read back asynchronously
@@ -3209,7 +3490,7 @@ int pcf_ensemble_solve_device(pcf_ensemble *e, const double *const *d_rhs, const
         PCF_CUDA_TRY(cudaEventRecord(h->ev[1], h->stream));
         if ((rc = assemble_device(h, dt[q], rayleigh_factor[q], prm->damp_horizontal_wind_on_rhs))) return rc;
         if (prm->preconditioner && !prm->multigrid && (rc = ensure_factors(h, deta_of(h, prm->dtau)))) return rc;
-        if (prm->multigrid && (rc = mg_prepare(h, prm, true))) return rc;
+        if (e->use_sp ? (rc = spectral_prepare(h)) : prm->multigrid ? (rc = mg_prepare(h, prm, true)) : 0) return rc;
         if (prm->autotune && (rc = autotune_handle(h, prm))) return rc;
         PCF_CUDA_TRY(cudaEventRecord(h->ev[2], h->stream));
         PCF_CUDA_TRY(cudaMemsetAsync(h->x64, 0, sizeof(double) * h->d.n, h->stream));
@@ -3225,7 +3506,7 @@ int pcf_ensemble_solve_device(pcf_ensemble *e, const double *const *d_rhs, const
     if (!e->exec || !e->key_valid || e->key_ci != ci || e->key_precond != prm->preconditioner ||
         e->key_pc_iters != prm->preconditioner_iterations || e->key_dtau != prm->dtau || e->key_mg != prm->multigrid ||
         e->key_mg_ci != prm->mg_coarse_iterations || e->key_mg_min != prm->mg_min_columns ||
-        e->key_mg_dtau != prm->mg_dtau || e->key_maxit != prm->poisson_iterations) {
+        e->key_mg_dtau != prm->mg_dtau || e->key_maxit != prm->poisson_iterations || e->key_sp != e->use_sp) {
         if ((rc = ensemble_capture(e, prm, ci))) return rc;
     }
     std::vector<double> bnorm(n), tol(n);
@@ -3251,12 +3532,12 @@ int pcf_ensemble_solve_device(pcf_ensemble *e, const double *const *d_rhs, const
             PCF_CUDA_TRY(cudaMemcpyAsync(h->scal32, &idle, sizeof(idle), cudaMemcpyHostToDevice, h->stream));
             continue;
         }
-        const LoopCfg c = ensemble_loop_cfg(h, prm);
+        const LoopCfg c = ensemble_loop_cfg(e, h, prm);
         const Work<float> w = work32_pi(h);
         k_to_float<<<vec_grid(h->d.n), 256, 0, h->stream>>>(h->w64, w.s, h->d.n, 1.0 / bnorm[q]);
         h->launches += 1;
         PCF_CUDA_TRY(cudaGetLastError());
-        if ((rc = run_start<float>(h, w, w.s, tol[q], maxit, c, 0, 1.0, bnorm[q], prm->inner_tolerance,
+        if ((rc = run_start<float>(h, w, w.s, loop_tolerance(tol[q], c), cap, c, 0, 1.0, bnorm[q], ru_delta(prm, c),
                                    prm->restart_interval)))
             return rc;
     }
@@ -3312,7 +3593,7 @@ int pcf_ensemble_solve_device(pcf_ensemble *e, const double *const *d_rhs, const
         PCF_CUDA_TRY(cudaStreamWaitEvent(h->stream, e->done, 0));
         const double *x = h->x64;
         if (active[q]) {
-            const LoopCfg c = ensemble_loop_cfg(h, prm);
+            const LoopCfg c = ensemble_loop_cfg(e, h, prm);
             const Work<float> w = work32_pi(h);
             float *xe = nullptr;
             RunOut ro;
@@ -3322,11 +3603,15 @@ int pcf_ensemble_solve_device(pcf_ensemble *e, const double *const *d_rhs, const
             reliable_bytes(h, ro.nupdates);
             res[q].status = ro.status;
             res[q].residual = res[q].true_residual = ro.nupdates > 0 ? ro.res : 1.0;
-            res[q].errflag = ro.converged ? 0 : 1;
-            if (!ro.converged && ro.status == PCF_EBREAKDOWN) {
+            const bool converged = ro.converged || (e->use_sp && ro.status == PCF_OK && res[q].residual <= tol[q]);
+            res[q].errflag = converged ? 0 : 1;
+            // (also one that the spectral preconditioner did not bring to convergence, with the V-cycle)
+            if (!converged && (ro.status == PCF_EBREAKDOWN || (ro.iters >= cap && cap < maxit))) {
                 pcf_result r2;
                 std::memset(&r2, 0, sizeof(r2));
-                if ((rc = krylov_solve(h, tolref[q], prm, &x, &r2))) return rc;
+                pcf_params again = *prm;
+                if (e->use_sp) again.poisson_iterations = std::max(1, maxit - ro.iters);
+                if ((rc = krylov_solve(h, tolref[q], &again, &x, &r2))) return rc;
                 r2.niter += res[q].niter;
                 r2.nrefine += res[q].nrefine;
                 res[q] = r2;

@@ -379,6 +379,13 @@ class PoissonSolver:
                    "pcf_apply_multigrid")
         return out
 
+    def apply_spectral(self, sin):
+        """The spectral preconditioner: pi = s / fcscal of the horizontally
+        averaged operator for the right-hand side sin (FP32 on the device)."""
+        out = np.zeros(self.dom.interior_shape)
+        _lib.check(self.lib.pcf_apply_spectral(self._h, _lib.dptr(_f64(sin)), _lib.dptr(out)), "pcf_apply_spectral")
+        return out
+
     def apply_bicgstab(self, rhs, tolref, namelist: PoissonNamelist):
         sol = np.zeros(self.dom.interior_shape)
         res = _lib.PcfResult()
