@@ -108,7 +108,7 @@ struct KrylovScalars {
     int nupdates;
     int restart_every;   // restart the Krylov recurrences (r0 = p = r_true) at every n-th update (0: never)
     int restart_now;     // set by FIN_RU_TRUE for the pending update
-    int pad2;
+    int passes;          // passes of the device-side loop (k_loop_continue)
 };
 
 // Finalisation performed by the last block of a fused reduction kernel.

@@ -146,7 +146,10 @@ static int pick_kc(long long xyblocks, int nz) {
     // at least 4 levels per block amortise the 5-plane prologue on large
     // grids; grids of a few x-y tiles (coarse multigrid levels, L2-resident)
     // are latency-bound, and one level per block shortens each block's chain
-    const long long kmin = xyblocks >= 16 ? 4 : 1;
+    // (and grids that 4-level blocks would leave with less than one block per
+    // SM: the FP64 residual at 64x64x32 ran 128 blocks in 23 us; at twice that
+    // bound the 128x96x48 grid's 288 blocks lost 7 %)
+    const long long kmin = xyblocks >= 16 && xyblocks * ((nz + 3) / 4) >= num_sms() ? 4 : 1;
     if (kc < kmin) kc = kmin;
     if (kc > nz) kc = nz;
     while (kc < nz && xyblocks * ((nz + kc - 1) / kc) > kMaxPartials) kc = std::min<long long>(2 * kc, nz);
@@ -1246,6 +1249,7 @@ static int mg_prepare(pcf_handle *h, const pcf_params *prm, bool ensemble = fals
 // Iterations a spectral solve gets to converge (4-10 on every grid tried); one
 // that has not by then goes on with the V-cycle from its last FP64 residual.
 constexpr int kSpectralIterations = 24;
+constexpr int kEnsembleSpectralBatch = 1;  // iterations per pass of the ensemble's loop
 constexpr int kSpectralMaxLevels = 512;  // column solves: 32 runs of at most 16 levels
 
 struct SpectralState {
@@ -1689,6 +1693,68 @@ struct GraphCache {
     std::vector<GraphEntry> entries;
 };
 
+// Last kernel of a device-side loop's body: another pass until the run is done.
+__global__ void k_loop_continue(KrylovScalars *s, cudaGraphConditionalHandle cond) {
+    s->passes += 1;
+    cudaGraphSetConditional(cond, !s->done && s->passes <= s->maxit ? 1u : 0u);
+}
+
+// The whole iteration as one graph: a conditional WHILE node around one
+// iteration.  Spectral runs take 4-6 iterations; issued in batches they left
+// up to 7 iterations of launches that return at once (2-27 us each, by grid
+// size) and waited for the host's look at the status word.  *out is null
+// where the driver has no conditional nodes.
+static int loop_graph(pcf_handle *h, const Work<float> &w, const LoopCfg &c, cudaGraphExec_t *out,
+                      long long *launches) {
+    *out = nullptr;
+    cudaGraph_t g = nullptr;
+    PCF_CUDA_TRY(cudaGraphCreate(&g, 0));
+    cudaGraphConditionalHandle cond;
+    cudaGraphNodeParams cp = {};
+    cudaGraphNode_t node;
+    cudaError_t e = cudaGraphConditionalHandleCreate(&cond, g, 1, cudaGraphCondAssignDefault);
+    if (e == cudaSuccess) {
+        cp.type = cudaGraphNodeTypeConditional;
+        cp.conditional.handle = cond;
+        cp.conditional.type = cudaGraphCondTypeWhile;
+        cp.conditional.size = 1;
+        e = cudaGraphAddNode(&node, g, nullptr, 0, &cp);
+    }
+    if (e != cudaSuccess) {
+        cudaGetLastError();
+        cudaGraphDestroy(g);
+        return PCF_OK;
+    }
+    e = cudaStreamBeginCaptureToGraph(h->stream, cp.conditional.phGraph_out[0], nullptr, nullptr, 0,
+                                      cudaStreamCaptureModeThreadLocal);
+    if (e != cudaSuccess) {
+        cudaGraphDestroy(g);
+        return pcf_set_cuda_error(e);
+    }
+    const long long l0 = h->launches;
+    const int rc = bicgstab_iteration<float>(h, w, c);
+    *launches = h->launches - l0 + 1;
+    h->launches = l0;  // captured, not launched
+    if (!rc) {
+        k_loop_continue<<<1, 1, 0, h->stream>>>(w.scal, cond);
+        e = cudaGetLastError();
+    }
+    cudaGraph_t body = nullptr;
+    const cudaError_t ee = cudaStreamEndCapture(h->stream, &body);
+    if (rc || e != cudaSuccess || ee != cudaSuccess) {
+        cudaGraphDestroy(g);
+        if (rc) return rc;
+        return pcf_set_cuda_error(e != cudaSuccess ? e : ee);
+    }
+    e = cudaGraphInstantiate(out, g, 0);
+    cudaGraphDestroy(g);
+    if (e != cudaSuccess) {
+        *out = nullptr;
+        return pcf_set_cuda_error(e);
+    }
+    return PCF_OK;
+}
+
 template <typename T>
 static int batch_graph(pcf_handle *h, const Work<T> &w, const LoopCfg &c, const GraphKey &key,
                        cudaGraphExec_t *out) {
@@ -1699,6 +1765,16 @@ static int batch_graph(pcf_handle *h, const Work<T> &w, const LoopCfg &c, const 
             h->graph_launches = e.launches;
             return PCF_OK;
         }
+    if constexpr (sizeof(T) == 4) {
+        if (key.batch == 0) {  // the device-side loop
+            long long nl = 0;
+            const int rc = loop_graph(h, w, c, out, &nl);
+            if (rc || !*out) return rc;
+            h->gcache->entries.push_back({key, *out, nl});
+            h->graph_launches = nl;
+            return PCF_OK;
+        }
+    }
     const long long l0 = h->launches;
     PCF_CUDA_TRY(cudaStreamBeginCapture(h->stream, cudaStreamCaptureModeThreadLocal));
     int rc = PCF_OK;
@@ -1735,7 +1811,8 @@ static void clear_graphs(pcf_handle *h) {
 // r0 = r = p = b, x = 0 (apply_bicgstab!.jl:44-67).
 template <typename T>
 static int run_start(pcf_handle *h, const Work<T> &w, const T *b, double tol, int maxit, const LoopCfg &c,
-                     int hist_off, double hist_scale, double bnorm64, double ru_delta, int restart_every) {
+                     int hist_off, double hist_scale, double bnorm64, double ru_delta, int restart_every,
+                     double start) {
     KrylovScalars init;
     std::memset(&init, 0, sizeof(init));
     init.tol = tol;
@@ -1749,6 +1826,11 @@ static int run_start(pcf_handle *h, const Work<T> &w, const T *b, double tol, in
     init.bnorm64 = bnorm64;
     init.ru_delta = ru_delta;
     init.restart_every = restart_every;
+    // A spectral iteration leaves so little that the first drop counts from the
+    // start (relative residual `start`): FP32 holds the true residual to 1e-5 -
+    // 1e-7 of it, so an iteration past the first such drop is lost (256x256x128:
+    // recursive 8e-7 and 3e-9 after two and three iterations, true 7e-6 either way).
+    init.res_max = c.sp ? start : 0.0;
     PCF_CUDA_TRY(cudaMemcpyAsync(w.scal, &init, sizeof(init), cudaMemcpyHostToDevice, h->stream));
     PCF_CUDA_TRY(cudaMemsetAsync(w.v, 0, sizeof(T) * h->d.n, h->stream));
     h->launches += 1;
@@ -1804,9 +1886,20 @@ template <typename T>
 static int bicgstab_run(pcf_handle *h, const Work<T> &w, const T *b, double tol, int maxit, const LoopCfg &c,
                         int check_interval, bool precondition_unconverged, T **xout, RunOut *out,
                         int hist_off = 0, double hist_scale = 1.0, double bnorm64 = 0.0, double ru_delta = 0.0,
-                        int restart_every = 0) {
-    int rc0 = run_start<T>(h, w, b, tol, maxit, c, hist_off, hist_scale, bnorm64, ru_delta, restart_every);
+                        int restart_every = 0, double start = 0.0) {
+    int rc0 = run_start<T>(h, w, b, tol, maxit, c, hist_off, hist_scale, bnorm64, ru_delta, restart_every, start);
     if (rc0) return rc0;
+    if (c.sp && !h->prof_on) {
+        cudaGraphExec_t loop = nullptr;
+        const int rc = batch_graph<T>(h, w, c, graph_key(h, (int)sizeof(T), c, w.post != nullptr, 0), &loop);
+        if (rc) return rc;
+        if (loop) {
+            PCF_CUDA_TRY(cudaGraphLaunch(loop, h->stream));
+            const int rf = run_finish<T>(h, w, c, precondition_unconverged, hist_off, xout, out);
+            h->launches += h->graph_launches * std::max(1, out->iters);
+            return rf;
+        }
+    }
     if (check_interval < 1) check_interval = 16;
     // Iterations are issued in batches of check_interval; a batch is a CUDA
     // graph (captured once per handle and loop configuration) unless per-launch
@@ -2934,7 +3027,7 @@ static int krylov_solve(pcf_handle *h, double tolref, const pcf_params *prm, con
                                                      : cm.sp       ? kSpectralIterations
                                                                    : maxit);
         rc = bicgstab_run<float>(h, w, w.s, loop_tolerance(tol, cm), cap, cm, prm->check_interval, false, &e, &ro, res->niter, 1.0,
-                                 b_norm, ru_delta(prm, cm), prm->restart_interval);
+                                 b_norm, ru_delta(prm, cm), prm->restart_interval, rel);
         if (rc) return rc;
         res->niter += ro.iters;
         res->nrefine += ro.nupdates;
@@ -3468,11 +3561,12 @@ int pcf_ensemble_solve_device(pcf_ensemble *e, const double *const *d_rhs, const
         (prm->multigrid && !prm->preconditioner))
         return PCF_EINVAL;
     PCF_CUDA_TRY(cudaSetDevice(e->device));
-    const int ci = prm->check_interval < 1 ? 16 : prm->check_interval;
     const int maxit = prm->poisson_iterations;
     int rc;
     e->use_sp = true;
     for (int q = 0; q < n; ++q) e->use_sp = e->use_sp && spectral_applies(e->m[q], prm);
+    // spectral members take 4-6 iterations: a longer batch is mostly launches of finished members
+    const int ci = e->use_sp ? kEnsembleSpectralBatch : prm->check_interval < 1 ? 16 : prm->check_interval;
     const int cap = e->use_sp ? std::min(maxit, kSpectralIterations) : maxit;
     PCF_CUDA_TRY(cudaEventRecord(e->t0, e->origin));
     // setup on every member's stream: inputs, assembly, pivots, multigrid
@@ -3538,7 +3632,7 @@ int pcf_ensemble_solve_device(pcf_ensemble *e, const double *const *d_rhs, const
         h->launches += 1;
         PCF_CUDA_TRY(cudaGetLastError());
         if ((rc = run_start<float>(h, w, w.s, loop_tolerance(tol[q], c), cap, c, 0, 1.0, bnorm[q], ru_delta(prm, c),
-                                   prm->restart_interval)))
+                                   prm->restart_interval, 1.0)))
             return rc;
     }
     for (int q = 0; q < n; ++q) {
