@@ -559,6 +559,13 @@ static int apply_total(pcf_handle *h, const StencilArgs<T> &a, bool diff) {
     return launch_stencil<T, false, EPI>(h, a);
 }
 
+// Grids of at most this many columns take the split sweep (k_thomas_split),
+// larger ones the column-per-thread sweep, which fills the GPU by itself there
+// (192x192x96 in FP32: 34 us, split 63 us).  Solves with the reference
+// preconditioner, column per thread -> split: 96x96x48 in FP64 30.2 -> 22.6 ms
+// (a sweep about 20 -> 8 us), 128x96x48 mixed 32.2 -> 27.2 ms.
+constexpr int kSplitThomasColumns = 16384;
+
 template <typename T, int MODE>
 static int launch_thomas(pcf_handle *h, const ThomasArgs<T> &a, int tag = -1) {
     const int bs = 128;
@@ -566,7 +573,25 @@ static int launch_thomas(pcf_handle *h, const ThomasArgs<T> &a, int tag = -1) {
     const int words = (MODE == TH_B || MODE == TH_T ? 1 : (MODE == TH_SUPD ? 3 : 4)) + 6;
     ProfScope ps(h, tag >= 0 ? tag : sizeof(T) == 4 ? PCF_PROF_THOMAS32 : PCF_PROF_THOMAS64,
                  (double)words * sizeof(T) * (double)a.n);
-    k_thomas<T, MODE><<<(a.plane + bs - 1) / bs, bs, 0, h->stream>>>(a);
+    // threads per column: runs of at most 8 levels, blocks of at most 1024
+    // threads (512 in FP64, whose runs need more registers)
+    constexpr int most = sizeof(T) == 4 ? 32 : 16;
+    int lpc = 2;
+    while (lpc < most && (a.nz + lpc - 1) / lpc > 8) lpc *= 2;
+    if (a.plane <= kSplitThomasColumns && (a.nz + lpc - 1) / lpc <= 8 && a.nz > 8) {
+        const unsigned grid = (unsigned)((a.plane + 31) / 32);
+        switch (lpc) {
+            case 2: k_thomas_split<T, MODE, 2><<<grid, dim3(32, 2), 0, h->stream>>>(a); break;
+            case 4: k_thomas_split<T, MODE, 4><<<grid, dim3(32, 4), 0, h->stream>>>(a); break;
+            case 8: k_thomas_split<T, MODE, 8><<<grid, dim3(32, 8), 0, h->stream>>>(a); break;
+            case 16: k_thomas_split<T, MODE, 16><<<grid, dim3(32, 16), 0, h->stream>>>(a); break;
+            default:
+                if constexpr (most == 32) k_thomas_split<T, MODE, 32><<<grid, dim3(32, 32), 0, h->stream>>>(a);
+                break;
+        }
+    } else {
+        k_thomas<T, MODE><<<(a.plane + bs - 1) / bs, bs, 0, h->stream>>>(a);
+    }
     PCF_CUDA_TRY(cudaGetLastError());
     return PCF_OK;
 }
@@ -784,29 +809,6 @@ __global__ void k_float_to_bf16(const float *__restrict__ a, __nv_bfloat16 *__re
         b[i] = __float2bfloat16_rn(a[i]);
 }
 
-// Coarse levels with few columns: k_thomas_split (runs of at most 8 levels,
-// up to 32 threads per column); otherwise the column-per-thread sweep.
-constexpr int kSplitThomasColumns = 16384;
-
-template <int MODE>
-static int mg_thomas(pcf_handle *h, const MgLevel &L, const ThomasArgs<float> &a, int tag) {
-    int lpc = 1;
-    while (lpc < 32 && (a.nz + lpc - 1) / lpc > 8) lpc *= 2;
-    if (L.d.plane > kSplitThomasColumns || (a.nz + lpc - 1) / lpc > 8 || a.post != nullptr || lpc < 2)
-        return launch_thomas<float, MODE>(h, a, tag);
-    ProfScope ps(h, tag, 6.0 * 4 * (double)a.n);
-    const unsigned grid = (unsigned)((a.plane + 31) / 32);
-    switch (lpc) {
-        case 2: k_thomas_split<MODE, 2><<<grid, dim3(32, 2), 0, h->stream>>>(a); break;
-        case 4: k_thomas_split<MODE, 4><<<grid, dim3(32, 4), 0, h->stream>>>(a); break;
-        case 8: k_thomas_split<MODE, 8><<<grid, dim3(32, 8), 0, h->stream>>>(a); break;
-        case 16: k_thomas_split<MODE, 16><<<grid, dim3(32, 16), 0, h->stream>>>(a); break;
-        default: k_thomas_split<MODE, 32><<<grid, dim3(32, 32), 0, h->stream>>>(a); break;
-    }
-    PCF_CUDA_TRY(cudaGetLastError());
-    return PCF_OK;
-}
-
 static ThomasArgs<float> mg_targs(const MgLevel &L, const float *fac, const float *in, float *out,
                                   const KrylovScalars *guard) {
     ThomasArgs<float> ta;
@@ -898,7 +900,7 @@ static int mg_pseudo_step(pcf_handle *h, const MgLevel &L, const float *coef, co
     if (rc) return rc;
     ThomasArgs<float> ta = mg_targs(L, fac, out, out, guard);
     ta.post = post;
-    return tag == PCF_PROF_MG ? mg_thomas<TH_T>(h, L, ta, tag) : launch_thomas<float, TH_T>(h, ta);
+    return launch_thomas<float, TH_T>(h, ta, tag == PCF_PROF_MG ? tag : -1);
 }
 
 // The coarse part of the cycle from level l = m.fused_from down, as one
@@ -956,7 +958,7 @@ static int mg_cycle(pcf_handle *h, int l, const KrylovScalars *guard, float **re
     if (l == m.fused_from) return mg_coarse_launch(h, l, guard, result);
     const MgLevel &L = m.lv[l];
     const __nv_bfloat16 *c16 = m.bf16 ? L.coef16 : nullptr;  // level 1 only
-    int rc = mg_thomas<TH_B>(h, L, mg_targs(L, L.fac, L.b, L.s, guard), PCF_PROF_MG);
+    int rc = launch_thomas<float, TH_B>(h, mg_targs(L, L.fac, L.b, L.s, guard), PCF_PROF_MG);
     if (rc) return rc;
     if (l + 1 == (int)m.lv.size()) {
         float *cur = L.s, *oth = L.t;
