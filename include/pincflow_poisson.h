@@ -186,7 +186,7 @@ typedef struct {
 typedef struct pcf_handle pcf_handle;
 
 /* Grids of at most 2048 cells are solved by the reference FP64 BiCGSTAB in a
- * single thread block (all vectors in shared memory), whatever precision,
+ * single launch (one thread-block cluster), whatever precision,
  * multigrid and learned say: the solve is launch-latency bound there.
  * Fills *p with the reference defaults. */
 int pcf_params_default(pcf_params *p);

@@ -2828,7 +2828,7 @@ static int zero_guess_residual(pcf_handle *h, const double *b, double *rms) {
 }
 
 // Grids of at most kTinyMaxCells cells: the reference FP64 BiCGSTAB in one
-// thread block (pcf_tiny.cuh), whatever the precision and multigrid settings
+// thread-block cluster (pcf_tiny.cuh), whatever the precision and multigrid settings
 // (on such grids the solve is bound by launch latency, so neither reduced
 // precision nor the multigrid hierarchy pays off).  Convergence is tested on
 // the recursive residual as in the reference; the FP64 true residual is
@@ -2838,19 +2838,13 @@ static int tiny_solve(pcf_handle *h, double tol, const pcf_params *prm, const do
     const double deta = deta_of(h, prm->dtau);
     int rc;
     if (prm->preconditioner && (rc = ensure_factors(h, deta))) return rc;
-    static int attr_device = -1;
-    const size_t smem = sizeof(double) * kTinyVectors * (size_t)h->d.n;
-    if (attr_device != h->dims.device) {
-        PCF_CUDA_TRY(cudaFuncSetAttribute(k_tiny_bicgstab, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                          (int)(sizeof(double) * kTinyVectors * kTinyMaxCells)));
-        attr_device = h->dims.device;
-    }
     TinyArgs a;
     a.nx = h->d.nx;
     a.ny = h->d.ny;
     a.nz = h->d.nz;
     a.n = (int)h->d.n;
     a.plane = h->d.plane;
+    a.ncol = (h->d.plane + kTinyCluster - 1) / kTinyCluster;
     a.coef = h->coef64;
     a.fac = h->fac64;
     a.b = h->b64;
@@ -2865,8 +2859,27 @@ static int tiny_solve(pcf_handle *h, double tol, const pcf_params *prm, const do
     a.hist_cap = kHistCap;
     {
         ProfScope ps(h, PCF_PROF_APPLY64, 0.0);
-        k_tiny_bicgstab<<<1, kTinyThreads, smem, h->stream>>>(a);
-        PCF_CUDA_TRY(cudaGetLastError());
+        // one cell a thread where the columns share out evenly enough, else two or eight
+        const int cells = a.ncol * a.nz;
+        auto kern = cells <= kTinyThreads       ? k_tiny_bicgstab<1>
+                    : cells <= 2 * kTinyThreads ? k_tiny_bicgstab<2>
+                                                : k_tiny_bicgstab<8>;
+        const size_t smem = tiny_smem(a.ncol, a.nz);
+        if (smem > 48 * 1024)
+            PCF_CUDA_TRY(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+        cudaLaunchConfig_t cfg{};
+        cfg.gridDim = dim3(kTinyCluster);
+        cfg.blockDim = dim3(kTinyThreads);
+        cfg.dynamicSmemBytes = smem;
+        cfg.stream = h->stream;
+        cudaLaunchAttribute attr[1];
+        attr[0].id = cudaLaunchAttributeClusterDimension;
+        attr[0].val.clusterDim.x = kTinyCluster;
+        attr[0].val.clusterDim.y = 1;
+        attr[0].val.clusterDim.z = 1;
+        cfg.attrs = attr;
+        cfg.numAttrs = 1;
+        PCF_CUDA_TRY(cudaLaunchKernelEx(&cfg, kern, a));
     }
     PCF_CUDA_TRY(cudaMemcpyAsync(h->h_scal, h->scal64, sizeof(KrylovScalars), cudaMemcpyDeviceToHost, h->stream));
     PCF_CUDA_TRY(cudaStreamSynchronize(h->stream));
