@@ -224,6 +224,11 @@ struct pcf_handle {
     long long coef8_version;
     float *rfc32;        // 1 / fcscal on the interior
     double fac_deta;  // d_eta the factors were built with (NaN: none)
+    // 1: the current operator exists in flux form only (pcf_flux.cuh: the first
+    // planes of coef64 and coefB32), assembled with these arguments; the
+    // coefficient planes follow on demand (ensure_planes)
+    int flux_only, flux_damp;
+    double flux_dt, flux_rf;
     // FP64 Krylov vectors
     double *x64, *r64, *r064, *p64, *v64, *s64, *t64, *za64, *zb64, *b64, *w64;
     // FP32 Krylov vectors

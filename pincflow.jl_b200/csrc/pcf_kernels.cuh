@@ -1082,7 +1082,7 @@ __global__ void __launch_bounds__(256) k_dot(const T *__restrict__ a, const T *_
     reduce_finalize<1>(red, v);
 }
 
-// Reliable update, step 1: x64 += bnorm64 * fcscal * x32 (the FP32 iteration
+// Reliable update, step 1: x64 += bnorm64 * fcscal * x32 (fc null: x64 holds pi) (the FP32 iteration
 // solves for pi = s / fcscal with the right-hand side scaled by 1 / bnorm64);
 // x32 = 0.
 __global__ void __launch_bounds__(256) k_ru_fold(float *x32, double *x64, const double *__restrict__ fc, long long n,
@@ -1091,7 +1091,7 @@ __global__ void __launch_bounds__(256) k_ru_fold(float *x32, double *x64, const 
     const double sc = scal->bnorm64;
     for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < n;
          i += (long long)gridDim.x * blockDim.x) {
-        x64[i] += sc * fc[i] * (double)x32[i];
+        x64[i] += (fc ? sc * fc[i] : sc) * (double)x32[i];
         x32[i] = 0.0f;
     }
 }

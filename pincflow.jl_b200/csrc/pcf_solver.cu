@@ -21,6 +21,7 @@
 #include "pcf_kernels.cuh"
 #include "pcf_mg.cuh"
 #include "pcf_spectral.cuh"
+#include "pcf_flux.cuh"
 #include "pcf_tiny.cuh"
 
 namespace {
@@ -1267,15 +1268,18 @@ struct SpectralState {
 
 // Whether a solve may replace the V-cycle by the spectral preconditioner: the
 // V-cycle's own settings are the defaults (others ask for that V-cycle), no
-// learned stage (trained on the V-cycle), and extents the kernels take.
+// network takes part (trained on the V-cycle and the planes), and extents the
+// kernels take.
 static bool spectral_applies(const pcf_handle *h, const pcf_params *prm) {
     pcf_params def;
     pcf_params_default(&def);
     return prm->multigrid && prm->precision == PCF_PRECISION_MIXED && prm->preconditioner &&
            prm->mg_dtau == def.mg_dtau && prm->mg_coarse_iterations == def.mg_coarse_iterations &&
            prm->mg_min_columns == def.mg_min_columns && prm->mg_operator_bf16 == def.mg_operator_bf16 &&
-           prm->mg_smoother_fp8 == def.mg_smoother_fp8 && !((prm->learned & 2) && h->net) && !h->test_stall &&
-           h->d.nx <= kFftMaxLength && h->d.ny <= kFftMaxLength && h->d.nz <= kSpectralMaxLevels;
+           prm->mg_smoother_fp8 == def.mg_smoother_fp8 && !(prm->learned && h->net) && !h->test_stall &&
+           (!prm->preconditioner || prm->preconditioner_iterations >= 1) &&
+           h->d.nx <= kFftMaxLength && h->d.ny <= kFftMaxLength && h->d.nz <= kSpectralMaxLevels &&
+           h->d.n < (1LL << 29);  // the flux-form apply's 32-bit byte offsets
 }
 
 static void spectral_free(pcf_handle *h) {
@@ -1387,6 +1391,11 @@ static int spectral_create(pcf_handle *h) {
     return PCF_OK;
 }
 
+// Words per cell of a flux-form apply: the values, pi, the second operand, the output.
+static double flux_words(const pcf_handle *h) {
+    return (h->dims.model == PCF_MODEL_COMPRESSIBLE ? FX_N : FX_DG) + 3.0;
+}
+
 // Level means and pivots of the current operator.
 static int spectral_prepare(pcf_handle *h) {
     int rc;
@@ -1394,15 +1403,52 @@ static int spectral_prepare(pcf_handle *h) {
     SpectralState &s = *h->spec;
     if (s.version == h->op_version) return PCF_OK;
     const SpectralArgs &a = s.a;
-    ProfScope ps(h, PCF_PROF_ASSEMBLE, 7.0 * 4 * (double)h->d.n + 4.0 * a.nz * a.nkx * a.nky, 3);
+    ProfScope ps(h, PCF_PROF_ASSEMBLE, (h->flux_only ? 5.0 : 7.0) * 4 * (double)h->d.n + 4.0 * a.nz * a.nkx * a.nky, 3);
     const int nblk = std::max(1, std::min(kLevelBlocks, std::min((h->d.plane + 255) / 256, 16 * num_sms() / a.nz + 1)));
-    k_level_sums<<<dim3((unsigned)nblk, (unsigned)a.nz), 256, 0, h->stream>>>(h->coefB32, h->d.plane, h->d.n, s.part);
+    const dim3 gs((unsigned)nblk, (unsigned)a.nz);
+    if (h->flux_only)
+        k_flux_sums<<<gs, 256, 0, h->stream>>>(h->coefB32, a.nx, a.ny, a.n, (float)(0.5 / h->dx), (float)(0.5 / h->dy),
+                                               h->dims.model == PCF_MODEL_COMPRESSIBLE, s.part, kLevelBlocks,
+                                               kLevelSums);
+    else
+        k_level_sums<<<gs, 256, 0, h->stream>>>(h->coefB32, h->d.plane, h->d.n, s.part);
     k_level_means<<<(unsigned)((kLevelSums * a.nz + 127) / 128), 128, 0, h->stream>>>(s.part, nblk, h->d.plane, a.nz,
                                                                                        s.lev, s.lad, s.lad + a.nz);
     k_spec_pivots<<<(unsigned)((a.nkx * a.nky + 127) / 128), 128, 0, h->stream>>>(s.lev, a.nx, a.ny, a.nz, a.nkx,
                                                                                    a.nky, s.piv);
     PCF_CUDA_TRY(cudaGetLastError());
     s.version = h->op_version;
+    return PCF_OK;
+}
+
+// The operator in flux form applied to a.s (pi), with the fused sums of EPI.
+template <typename T, int EPI>
+static int flux_apply(pcf_handle *h, FluxArgs<T> a) {
+    a.f = sizeof(T) == 4 ? (const T *)h->coefB32 : (const T *)h->coef64;
+    a.nx = h->d.nx;
+    a.ny = h->d.ny;
+    a.nz = h->d.nz;
+    a.n = h->d.n;
+    a.rdx = 1.0 / h->dx;
+    a.rdy = 1.0 / h->dy;
+    a.rdz = 1.0 / h->dz;
+    a.diag = h->dims.model == PCF_MODEL_COMPRESSIBLE;
+    const long long gx = (a.nx + kFluxTX - 1) / kFluxTX, gy = (a.ny + kFluxTY - 1) / kFluxTY, xy = gx * gy;
+    if (gy > 65535) return PCF_ERANGE;
+    // levels per block: about 24 blocks per SM, so that the last of the 5
+    // resident waves matters little, and at least 4 levels, as each chunk
+    // evaluates one more; 2 on grids that leave the GPU mostly idle
+    const long long chunks = std::max<long long>(1, (24LL * num_sms() + xy - 1) / xy);
+    long long kc = std::max<long long>((a.nz + chunks - 1) / chunks, xy * ((a.nz + 3) / 4) < 4LL * num_sms() ? 2 : 4);
+    kc = std::min<long long>(kc, a.nz);
+    while (kc < a.nz && xy * ((a.nz + kc - 1) / kc) > kMaxPartials) kc = std::min<long long>(2 * kc, a.nz);
+    const long long gz = (a.nz + kc - 1) / kc;
+    if (xy * gz > kMaxPartials) return PCF_ERANGE;
+    ProfScope ps(h, a.guard_update ? PCF_PROF_RELIABLE : sizeof(T) == 4 ? PCF_PROF_APPLY32 : PCF_PROF_APPLY64,
+                 a.guard_update ? 0.0 : flux_words(h) * sizeof(T) * (double)a.n);
+    k_flux_apply<T, EPI><<<dim3((unsigned)gx, (unsigned)gy, (unsigned)gz), dim3(kFluxTX, kFluxTY), 0, h->stream>>>(
+        a, (int)kc);
+    PCF_CUDA_TRY(cudaGetLastError());
     return PCF_OK;
 }
 
@@ -1491,6 +1537,7 @@ struct LoopCfg {
     int reliable;  // fold into the FP64 solution and restart r from the true residual
     int mg = 0;    // multigrid V-cycle as the preconditioner (FP32 loop only)
     int sp = 0;    // spectral preconditioner (FP32 loop only)
+    int fx = 0;    // the operator in flux form (pcf_flux.cuh), x64 in pi
     int learned_pc = 0;  // learned stage after the preconditioner (FP32 loop only)
 };
 
@@ -1522,19 +1569,35 @@ static int learned_stage(pcf_handle *h, const Work<float> &w, const float *bvec,
 
 // Profiler bytes of the FP64 true-residual applies of `nupdates` reliable
 // updates: 25 coefficient planes + x + b + r words per cell.
-static void reliable_bytes(pcf_handle *h, int nupdates) {
+static void reliable_bytes(pcf_handle *h, int nupdates, double words = 28.0) {
     if (h->prof_on && h->prof && nupdates > 0)
-        h->prof_acc[PCF_PROF_RELIABLE].bytes += (double)nupdates * 28.0 * sizeof(double) * (double)h->d.n;
+        h->prof_acc[PCF_PROF_RELIABLE].bytes += (double)nupdates * words * sizeof(double) * (double)h->d.n;
 }
 
 // Reliable update (mixed precision): x64 += bnorm64 x32, r64 = b - A64 x64
 // with the FP64 convergence test, r32 = r64 / bnorm64, <r32, r0>.  The three
 // launches return at once unless the last FIN_RESID raised the update flag.
-static int reliable_update(pcf_handle *h) {
+// fx: the operator is in flux form and x64 holds pi (no fcscal).
+static int reliable_update(pcf_handle *h, bool fx) {
     KrylovScalars *sc = h->scal32;
     h->launches += 1;
-    k_ru_fold<<<vec_grid(h->d.n), 256, 0, h->stream>>>(h->x32, h->x64, h->fc64, h->d.n, sc);
+    k_ru_fold<<<vec_grid(h->d.n), 256, 0, h->stream>>>(h->x32, h->x64, fx ? nullptr : h->fc64, h->d.n, sc);
     PCF_CUDA_TRY(cudaGetLastError());
+    int rc;
+    if (fx) {
+        FluxArgs<double> f;
+        f.s = h->x64;
+        f.out = h->w64;
+        f.w1 = h->b64;
+        f.guard = sc;
+        f.guard_update = 1;
+        f.red = red(h, sc, FIN_RU_TRUE);
+        if ((rc = flux_apply<double, EPI_RESID>(h, f))) return rc;
+        h->launches += 1;
+        k_ru_convert<<<vec_grid(h->d.n), 256, 0, h->stream>>>(h->w64, h->r32, h->r032, h->d.n, red(h, sc, FIN_RU_RHO));
+        PCF_CUDA_TRY(cudaGetLastError());
+        return PCF_OK;
+    }
     StencilArgs<double> a;
     a.coef = h->coef64;
     a.s = h->x64;
@@ -1544,7 +1607,7 @@ static int reliable_update(pcf_handle *h) {
     a.guard = sc;
     a.guard_update = 1;
     a.red = red(h, sc, FIN_RU_TRUE);
-    int rc = launch_stencil<double, false, EPI_RESID>(h, a);
+    rc = launch_stencil<double, false, EPI_RESID>(h, a);
     if (rc) return rc;
     h->launches += 1;
     k_ru_convert<<<vec_grid(h->d.n), 256, 0, h->stream>>>(h->w64, h->r32, h->r032, h->d.n, red(h, sc, FIN_RU_RHO));
@@ -1581,7 +1644,20 @@ static int bicgstab_iteration(pcf_handle *h, const Work<T> &w, const LoopCfg &c)
     }
     if (rc) return rc;
     // v = A z; alpha = <r, r0> / <v, r0>
-    {
+    bool applied = false;
+    if constexpr (sizeof(T) == 4) {
+        if (c.fx) {
+            FluxArgs<float> fa;
+            fa.s = z;
+            fa.out = w.v;
+            fa.w1 = w.r0;
+            fa.red = red(h, w.scal, FIN_ALPHA);
+            fa.guard = w.scal;
+            if ((rc = flux_apply<float, EPI_DOT1>(h, fa))) return rc;
+            applied = true;
+        }
+    }
+    if (!applied) {
         StencilArgs<T> sa;
         sa.coef = w.coefT;
         sa.s = z;
@@ -1621,7 +1697,18 @@ static int bicgstab_iteration(pcf_handle *h, const Work<T> &w, const LoopCfg &c)
     }
     if (rc) return rc;
     // t = A z; omega = <t, s> / <t, t>
-    {
+    if constexpr (sizeof(T) == 4) {
+        if (c.fx) {
+            FluxArgs<float> fa;
+            fa.s = z;
+            fa.out = w.t;
+            fa.w1 = w.s;
+            fa.red = red(h, w.scal, FIN_OMEGA);
+            fa.guard = w.scal;
+            if ((rc = flux_apply<float, EPI_DOT2>(h, fa))) return rc;
+        }
+    }
+    if (!applied) {
         StencilArgs<T> sa;
         sa.coef = w.coefT;
         sa.s = z;
@@ -1661,7 +1748,7 @@ static int bicgstab_iteration(pcf_handle *h, const Work<T> &w, const LoopCfg &c)
         }
         PCF_CUDA_TRY(cudaGetLastError());
     }
-    if (c.reliable) return reliable_update(h);
+    if (c.reliable) return reliable_update(h, c.fx != 0);
     return PCF_OK;
 }
 
@@ -1677,7 +1764,7 @@ struct GraphKey {
     int tsize, precond, pc_iters, flex, reliable, pi, batch;
     double deta;
     int mg, mg_levels, mg_coarse_iters, mg_bf16;
-    int sp;           // spectral preconditioner
+    int sp;           // spectral preconditioner, flux-form operator
     const void *net;  // the learned stage's network (null: no stage)
     bool operator==(const GraphKey &o) const {
         return tsize == o.tsize && precond == o.precond && pc_iters == o.pc_iters && flex == o.flex &&
@@ -1880,7 +1967,7 @@ static GraphKey graph_key(const pcf_handle *h, int tsize, const LoopCfg &c, bool
     return GraphKey{tsize, c.precond, c.pc_iters, c.flex, c.reliable, pi, check_interval, c.deta, c.mg,
                     c.mg && h->mg ? (int)h->mg->lv.size() : 0, c.mg && h->mg ? h->mg->coarse_iters : 0,
                     c.mg && h->mg ? (int)h->mg->bf16 | (h->mg->lv[0].tmap8 ? 2 : 0) | (h->mg->fused_from + 1) << 2 : 0,
-                    c.sp, c.learned_pc ? (const void *)h->net : nullptr};
+                    c.sp | c.fx << 1, c.learned_pc ? (const void *)h->net : nullptr};
 }
 
 // A complete BiCGSTAB run: run_start, the iteration batches, run_finish.
@@ -1968,6 +2055,10 @@ __global__ void k_axpy_f2d(const float *__restrict__ e, double *__restrict__ x, 
     for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < n; i += (long long)gridDim.x * blockDim.x)
         x[i] += (double)e[i] * scale * (fc ? fc[i] : 1.0);
 }
+__global__ void k_mul(double *__restrict__ x, const double *__restrict__ f, long long n) {
+    for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < n; i += (long long)gridDim.x * blockDim.x)
+        x[i] *= f[i];
+}
 // pi = s / fcscal in FP32 (for the difference-form operator entry point)
 __global__ void k_to_pi(const double *__restrict__ s, const float *__restrict__ rfc, float *__restrict__ pi,
                         long long n) {
@@ -1980,16 +2071,20 @@ __global__ void k_coef_to_float(const double *__restrict__ a, float *__restrict_
 }
 // dpip = (1/dt) * s / sqrt(pbar^2 / rhobar) on the interior (solve_poisson!.jl:65-72);
 // dst is haloed with offsets (ox, oy, oz) and pitches (sx, sy), or compact.
-__global__ void k_unscale(const double *__restrict__ x, const double *__restrict__ pbar,
+// pi: x already holds s / sqrt(pbar^2 / rhobar).
+__global__ void k_unscale(const double *__restrict__ x, bool pi, const double *__restrict__ pbar,
                           const double *__restrict__ rhobar, double dtinv, int nx, int ny, int nz, int nbx, int nby,
                           int nbz, int nxx, int nyy, double *__restrict__ dst, int ox, int oy, int oz, int sx, int sy) {
     const long long n = (long long)nx * ny * nz;
     for (long long c = blockIdx.x * (long long)blockDim.x + threadIdx.x; c < n; c += (long long)gridDim.x * blockDim.x) {
         const unsigned cu = (unsigned)c, ux = (unsigned)nx, uy = (unsigned)ny;  // n < 2^31 (see k_build_diff)
         const int i = (int)(cu % ux), j = (int)((cu / ux) % uy), k = (int)(cu / (ux * uy));
-        const long long hh = (i + nbx) + (long long)nxx * ((j + nby) + (long long)nyy * (k + nbz));
-        const double pb = pbar[hh];
-        const double sol = x[c] / sqrt(pb * pb / rhobar[hh]);
+        double sol = x[c];
+        if (!pi) {
+            const long long hh = (i + nbx) + (long long)nxx * ((j + nby) + (long long)nyy * (k + nbz));
+            const double pb = pbar[hh];
+            sol = sol / sqrt(pb * pb / rhobar[hh]);
+        }
         dst[(i + ox) + (long long)sx * ((j + oy) + (long long)sy * (k + oz))] = dtinv * sol;
     }
 }
@@ -2044,6 +2139,8 @@ int pcf_params_default(pcf_params *p) {
     p->mg_smoother_fp8 = 0;
     return PCF_OK;
 }
+
+static int ensure_planes(pcf_handle *h);
 
 static int dalloc(pcf_handle *h, void **p, size_t bytes) {
     cudaError_t e = cudaMalloc(p, bytes);
@@ -2187,6 +2284,8 @@ int pcf_set_grid(pcf_handle *h, double dx, double dy, double dz, const double *j
                  const double *met23, const double *met33) {
     if (!h || !jac || !met13 || !met23 || !met33 || !(dx > 0) || !(dy > 0) || !(dz > 0)) return PCF_EINVAL;
     PCF_CUDA_TRY(cudaSetDevice(h->dims.device));
+    int rp = ensure_planes(h);  // of the operator assembled from the fields replaced here
+    if (rp) return rp;
     const size_t b = sizeof(double) * (size_t)h->nh;
     h->dx = dx;
     h->dy = dy;
@@ -2206,6 +2305,8 @@ int pcf_set_background(pcf_handle *h, const double *pbar, const double *rhobar, 
     if (!h || !pbar || !rhobar || !n2) return PCF_EINVAL;
     if (h->dims.model == PCF_MODEL_COMPRESSIBLE && !thetabar) return PCF_EINVAL;
     PCF_CUDA_TRY(cudaSetDevice(h->dims.device));
+    int rp = ensure_planes(h);  // of the operator assembled from the fields replaced here
+    if (rp) return rp;
     const size_t b = sizeof(double) * (size_t)h->nh;
     PCF_CUDA_TRY(cudaMemcpyAsync(h->pbar, pbar, b, cudaMemcpyHostToDevice, h->stream));
     PCF_CUDA_TRY(cudaMemcpyAsync(h->rhobar, rhobar, b, cudaMemcpyHostToDevice, h->stream));
@@ -2218,11 +2319,77 @@ int pcf_set_background(pcf_handle *h, const double *pbar, const double *rhobar, 
     return PCF_OK;
 }
 
+// The flux-form operator of levels [z0, z1).
+static int flux_build(pcf_handle *h, double dt, double rf, int damp_h, int z0, int z1) {
+    FluxBuildArgs a;
+    a.nx = h->d.nx;
+    a.ny = h->d.ny;
+    a.nz = h->d.nz;
+    a.nxx = h->nxx;
+    a.nyy = h->nyy;
+    a.nbx = h->dims.nbx;
+    a.nby = h->dims.nby;
+    a.nbz = h->dims.nbz;
+    a.model = h->dims.model;
+    a.damp_h = damp_h;
+    a.z0 = z0;
+    a.z1 = z1;
+    a.dt = dt;
+    a.rf = rf;
+    a.rdx = 1.0 / h->dx;
+    a.rdy = 1.0 / h->dy;
+    a.rdz = 1.0 / h->dz;
+    // Constants.jl:119-128
+    a.gamma = 1.4;
+    a.kappa = (1.4 - 1.0) / 1.4;
+    a.rsp = 287.0;
+    a.pref = 101325.0;
+    a.jac = h->jac;
+    a.met13 = h->met13;
+    a.met23 = h->met23;
+    a.met33 = h->met33;
+    a.pbar = h->pbar;
+    a.rhobar = h->rhobar;
+    a.thetabar = h->thetabar;
+    a.n2 = h->n2;
+    a.rho = h->rho;
+    a.betar = h->betar;
+    a.p = h->p;
+    a.rfch = h->rfch;
+    a.f64 = h->coef64;
+    a.f32 = h->coefB32;
+    a.uneven = h->ticket + 2;
+    if (z0 == 0) PCF_CUDA_TRY(cudaMemsetAsync(a.uneven, 0, sizeof(unsigned), h->stream));
+    const dim3 g((unsigned)((a.nx + 63) / 64), (unsigned)((a.ny + 3) / 4), (unsigned)(z1 - z0));
+    // 11 haloed fields read, 10 values written in FP64 and FP32
+    ProfScope ps(h, PCF_PROF_ASSEMBLE, (11.0 * 8 + 10.0 * 12) * (double)h->d.plane * (z1 - z0));
+    k_flux_build<<<g, dim3(64, 4), 0, h->stream>>>(a);
+    PCF_CUDA_TRY(cudaGetLastError());
+    return PCF_OK;
+}
+
 // Assembles z-chunks [c0, c1) (c1 < 0: to the top); the operator is set
-// once the last chunk is queued.
-static int assemble_chunks(pcf_handle *h, double dt, double rf, int damp_h, int c0, int c1) {
+// once the last chunk is queued.  flux: in flux form only (spectral solves).
+static int assemble_chunks(pcf_handle *h, double dt, double rf, int damp_h, int c0, int c1, bool flux = false) {
     const int nchunks = (h->d.nz + pcf_assemble_chunk_levels() - 1) / pcf_assemble_chunk_levels();
     if (c1 < 0 || c1 > nchunks) c1 = nchunks;
+    if (flux) {
+        const int levels = pcf_assemble_chunk_levels();
+        if (c0 < c1) {
+            const int rc = flux_build(h, dt, rf, damp_h, c0 * levels, std::min(h->d.nz, c1 * levels));
+            if (rc) return rc;
+        }
+        if (c1 == nchunks) {
+            h->operator_set = 1;
+            h->op_version += 1;
+            h->fac_deta = std::nan("");
+            h->flux_only = 1;
+            h->flux_dt = dt;
+            h->flux_rf = rf;
+            h->flux_damp = damp_h;
+        }
+        return PCF_OK;
+    }
     // 11 haloed fields read; 25 FP64, 25 FP32, 25 difference-form FP32 (and
     // 25 BF16) planes, fcscal and 1 / fcscal written per cell
     {
@@ -2234,13 +2401,22 @@ static int assemble_chunks(pcf_handle *h, double dt, double rf, int damp_h, int 
     if (c1 == nchunks) {
         h->operator_set = 1;
         h->op_version += 1;
+        h->flux_only = 0;
     }
     return PCF_OK;
 }
 
-static int assemble_device(pcf_handle *h, double dt, double rf, int damp_h) {
+static int assemble_device(pcf_handle *h, double dt, double rf, int damp_h, bool flux = false) {
     if (!h->grid_set || !h->background_set) return PCF_ENOTREADY;
-    return assemble_chunks(h, dt, rf, damp_h, 0, -1);
+    return assemble_chunks(h, dt, rf, damp_h, 0, -1, flux);
+}
+
+// The coefficient planes of the current operator, where a spectral solve left
+// it in flux form (its inputs are the handle's own rho, betar, p, grid and
+// background until they are next replaced).
+static int ensure_planes(pcf_handle *h) {
+    if (!h->flux_only) return PCF_OK;
+    return assemble_chunks(h, h->flux_dt, h->flux_rf, h->flux_damp, 0, -1);
 }
 
 int pcf_compute_operator(pcf_handle *h, const double *rho, const double *betar, const double *p, double dt,
@@ -2277,6 +2453,7 @@ int pcf_set_operator(pcf_handle *h, const double *coef) {
     }
     h->operator_set = 1;
     h->op_version += 1;
+    h->flux_only = 0;
     h->fac_deta = std::nan("");
     int rc = build_diff(h, h->background_set);
     if (rc) return rc;
@@ -2298,7 +2475,8 @@ int pcf_apply_operator(pcf_handle *h, const double *sin_, double *ls, int mode, 
     if (!h || !sin_ || !ls || (mode != PCF_TOTAL && mode != PCF_HORIZONTAL)) return PCF_EINVAL;
     if (!h->operator_set) return PCF_ENOTREADY;
     PCF_CUDA_TRY(cudaSetDevice(h->dims.device));
-    int rc;
+    int rc = ensure_planes(h);
+    if (rc) return rc;
     if (precision == PCF_PRECISION_MIXED) {
         // the FP32 difference-form operator of the mixed solve, applied to s
         if (mode != PCF_TOTAL) return PCF_EINVAL;
@@ -2353,8 +2531,8 @@ int pcf_apply_preconditioner(pcf_handle *h, const double *sin_, double *sout, co
     if (!h->operator_set) return PCF_ENOTREADY;
     PCF_CUDA_TRY(cudaSetDevice(h->dims.device));
     const double deta = deta_of(h, prm->dtau);
-    int rc = ensure_factors(h, deta);
-    if (rc) return rc;
+    int rc = ensure_planes(h);
+    if (rc || (rc = ensure_factors(h, deta))) return rc;
     if (precision == PCF_PRECISION_FP32) {
         if ((rc = upload_vec(h, sin_, h->b64, h->s32))) return rc;
         float *z = nullptr;
@@ -2378,8 +2556,8 @@ int pcf_multigrid_levels(pcf_handle *h, const pcf_params *prm, int cap, int *nle
     if (!h || !prm || !nlevels || cap < 0 || (cap > 0 && !dims)) return PCF_EINVAL;
     if (!h->operator_set) return PCF_ENOTREADY;
     PCF_CUDA_TRY(cudaSetDevice(h->dims.device));
-    int rc = mg_prepare(h, prm);
-    if (rc) return rc;
+    int rc = ensure_planes(h);
+    if (rc || (rc = mg_prepare(h, prm))) return rc;
     const int nl = (int)h->mg->lv.size();
     *nlevels = nl;
     for (int l = 0; l < nl && l < cap; ++l) {
@@ -2394,6 +2572,8 @@ int pcf_multigrid_levels(pcf_handle *h, const pcf_params *prm, int cap, int *nle
 int pcf_multigrid_operator(pcf_handle *h, int level, double *coef) {
     if (!h || !coef || !h->mg || level < 0 || level >= (int)h->mg->lv.size()) return PCF_EINVAL;
     PCF_CUDA_TRY(cudaSetDevice(h->dims.device));
+    const int rc = ensure_planes(h);
+    if (rc) return rc;
     const MgLevel &L = h->mg->lv[level];
     const long long m = L.d.n * PCF_NCOEF;
     if (level == 0) {
@@ -2412,8 +2592,8 @@ int pcf_apply_multigrid(pcf_handle *h, const double *sin_, double *sout, const p
     if (!h || !sin_ || !sout || !prm) return PCF_EINVAL;
     if (!h->operator_set) return PCF_ENOTREADY;
     PCF_CUDA_TRY(cudaSetDevice(h->dims.device));
-    int rc = mg_prepare(h, prm);
-    if (rc) return rc;
+    int rc = ensure_planes(h);
+    if (rc || (rc = mg_prepare(h, prm))) return rc;
     if ((rc = upload_vec(h, sin_, h->b64, h->s32))) return rc;
     float *z = nullptr;
     rc = mg_precond<TH_B>(h, work32(h), h->s32, nullptr, &z, h->za32, h->zb32, nullptr);
@@ -2430,8 +2610,8 @@ int pcf_apply_spectral(pcf_handle *h, const double *sin_, double *sout) {
     if (!h->operator_set) return PCF_ENOTREADY;
     if (h->d.nx > kFftMaxLength || h->d.ny > kFftMaxLength || h->d.nz > kSpectralMaxLevels) return PCF_ERANGE;
     PCF_CUDA_TRY(cudaSetDevice(h->dims.device));
-    int rc = spectral_prepare(h);
-    if (rc) return rc;
+    int rc = ensure_planes(h);
+    if (rc || (rc = spectral_prepare(h))) return rc;
     if ((rc = upload_vec(h, sin_, h->b64, h->s32))) return rc;
     if ((rc = spectral_precond<TH_B>(h, work32(h), h->s32, h->za32, nullptr))) return rc;
     k_to_double<<<vec_grid(h->d.n), 256, 0, h->stream>>>(h->za32, h->w64, h->d.n);
@@ -2815,13 +2995,15 @@ static int true_residual(pcf_handle *h, const double *b, const double *x, double
 
 // The FP64 residual of the zero initial guess, r64 = b (into w64, as
 // true_residual leaves it), and its RMS: one pass over b instead of an
-// operator apply.
-static int zero_guess_residual(pcf_handle *h, const double *b, double *rms) {
+// operator apply.  uneven (may be null): k_flux_build's finding on the halos.
+static int zero_guess_residual(pcf_handle *h, const double *b, double *rms, unsigned *uneven) {
     k_copy_sumsq<<<vec_grid(h->d.n), 256, 0, h->stream>>>(b, h->w64, h->d.n, red(h, nullptr, FIN_STORE, h->dot_out));
     h->launches += 1;
     PCF_CUDA_TRY(cudaGetLastError());
     double rr = 0;
     PCF_CUDA_TRY(cudaMemcpyAsync(&rr, h->dot_out, sizeof(double), cudaMemcpyDeviceToHost, h->stream));
+    if (uneven)
+        PCF_CUDA_TRY(cudaMemcpyAsync(uneven, h->ticket + 2, sizeof(unsigned), cudaMemcpyDeviceToHost, h->stream));
     PCF_CUDA_TRY(cudaStreamSynchronize(h->stream));
     *rms = std::sqrt(rr / (double)h->d.n);
     return PCF_OK;
@@ -2925,9 +3107,13 @@ static double loop_tolerance(double tol, const LoopCfg &c) { return c.sp ? 0.1 *
 
 // Solves A x = b64 (device) according to prm; the solution ends in *xres
 // (a device FP64 buffer owned by the handle).
-// spectral: the caller lets the spectral preconditioner stand in for the V-cycle (spectral_applies).
+// pi: null, or where a caller that let the spectral preconditioner stand in for
+// the V-cycle (flux_only, the operator assembled in flux form) is told whether
+// *xres holds pi = s / fcscal.
 static int krylov_solve(pcf_handle *h, double tolref, const pcf_params *prm, const double **xres, pcf_result *res,
-                        bool spectral = false) {
+                        bool *pi = nullptr) {
+    bool spectral = pi != nullptr && h->flux_only;
+    if (pi) *pi = false;
     const double tol = prm->tolerance_is_relative ? prm->tolerance : prm->tolerance / tolref;  // :49-53
     LoopCfg c;
     c.precond = prm->preconditioner;
@@ -2938,8 +3124,9 @@ static int krylov_solve(pcf_handle *h, double tolref, const pcf_params *prm, con
     if (c.precond && c.pc_iters < 1) return PCF_EINVAL;
     // the multigrid preconditioner runs in the FP32 loop of the mixed solve only
     if (prm->multigrid && (prm->precision != PCF_PRECISION_MIXED || !c.precond)) return PCF_EINVAL;
-    if (h->d.n <= kTinyMaxCells) return tiny_solve(h, tol, prm, xres, res);
     int rc;
+    if (!spectral && (rc = ensure_planes(h))) return rc;
+    if (h->d.n <= kTinyMaxCells) return tiny_solve(h, tol, prm, xres, res);
     // (the multigrid mixed solve builds the pivots of its own d_eta in mg_prepare)
     if (c.precond && !prm->multigrid && (rc = ensure_factors(h, c.deta))) return rc;
     const int maxit = prm->poisson_iterations;
@@ -2968,7 +3155,8 @@ static int krylov_solve(pcf_handle *h, double tolref, const pcf_params *prm, con
     // x64 accumulates the correction; r64 = b - A x64 is the FP64 true residual.
     PCF_CUDA_TRY(cudaMemsetAsync(h->x64, 0, sizeof(double) * h->d.n, h->stream));
     double rnorm = 0;
-    if ((rc = zero_guess_residual(h, h->b64, &rnorm))) return rc;
+    unsigned uneven = 0;
+    if ((rc = zero_guess_residual(h, h->b64, &rnorm, spectral ? &uneven : nullptr))) return rc;
     const double b_norm = rnorm;
     res->b_norm = b_norm;
     if ((prm->learned & 1) && h->net && b_norm > 0 && std::isfinite(b_norm)) {
@@ -3004,16 +3192,27 @@ static int krylov_solve(pcf_handle *h, double tolref, const pcf_params *prm, con
     cm.flex = 1;
     cm.reliable = 1;
     auto use_vcycle = [&]() -> int {
+        int r;
         cm.sp = 0;
-        const int r = mg_prepare(h, prm);
-        if (r) return r;
+        if (cm.fx) {  // from pi and the flux form to s and the planes
+            cm.fx = 0;
+            *pi = false;
+            if ((r = ensure_planes(h))) return r;
+            k_mul<<<vec_grid(h->d.n), 256, 0, h->stream>>>(h->x64, h->fc64, h->d.n);
+            h->launches += 1;
+            PCF_CUDA_TRY(cudaGetLastError());
+        }
+        if ((r = mg_prepare(h, prm))) return r;
         cm.mg = 1;
         cm.deta = h->mg->lv[0].deta;
         return PCF_OK;
     };
-    if (spectral && spectral_applies(h, prm)) {
+    if (spectral) {
+        // halo columns that are not the periodic image: the planes tell them apart
+        if (uneven && (rc = ensure_planes(h))) return rc;
         if ((rc = spectral_prepare(h))) return rc;
         cm.sp = 1;
+        cm.fx = *pi = !uneven;
         cm.deta = 0;
     } else if (prm->multigrid && (rc = use_vcycle())) {
         return rc;
@@ -3046,7 +3245,7 @@ static int krylov_solve(pcf_handle *h, double tolref, const pcf_params *prm, con
         if (rc) return rc;
         res->niter += ro.iters;
         res->nrefine += ro.nupdates;
-        reliable_bytes(h, ro.nupdates);
+        reliable_bytes(h, ro.nupdates, cm.fx ? flux_words(h) : 28.0);
         if (ro.nupdates > 0) rel = ro.res;
         if (ro.converged || (cm.sp && ro.status == PCF_OK && rel <= tol)) break;
         const bool stalled = (cm.learned_pc || cm.sp) && ro.iters >= cap && res->niter < maxit;
@@ -3093,18 +3292,26 @@ static float elapsed(cudaEvent_t a, cudaEvent_t b) {
     return ms;
 }
 
+// A solve of this handle with these settings is spectral (and its operator
+// assembled in flux form only).
+static bool spectral_solve(const pcf_handle *h, const pcf_params *prm) {
+    return spectral_applies(h, prm) && h->d.n > kTinyMaxCells;
+}
+
 // rhs_ready: an event the solve waits for after the assembly (the right-hand
 // side's upload on the copy stream), or null.  assembled: the caller queued
 // the assembly (and recorded ev[1] where it starts).
 static int solve_common(pcf_handle *h, double dt, double rf, double tolref, const pcf_params *prm, pcf_result *res,
-                        const double **x, cudaEvent_t rhs_ready = nullptr, bool assembled = false) {
+                        const double **x, bool *pi, cudaEvent_t rhs_ready = nullptr, bool assembled = false) {
     // solve_poisson!.jl:52-54
     if (dt == 0.0) return PCF_EINVAL;
     int rc;
     if (!assembled) PCF_CUDA_TRY(cudaEventRecord(h->ev[1], h->stream));
     {
         NvtxScope r("pcf assemble");
-        if (!assembled && (rc = assemble_device(h, dt, rf, prm->damp_horizontal_wind_on_rhs))) return rc;
+        if (!assembled &&
+            (rc = assemble_device(h, dt, rf, prm->damp_horizontal_wind_on_rhs, spectral_solve(h, prm))))
+            return rc;
         // the multigrid mixed solve builds the pivots of its own d_eta (mg_prepare)
         const bool mg = prm->multigrid && prm->precision == PCF_PRECISION_MIXED;
         if (prm->preconditioner && !mg && (rc = ensure_factors(h, deta_of(h, prm->dtau)))) return rc;
@@ -3113,7 +3320,7 @@ static int solve_common(pcf_handle *h, double dt, double rf, double tolref, cons
     PCF_CUDA_TRY(cudaEventRecord(h->ev[2], h->stream));
     {
         NvtxScope r("pcf krylov");
-        if ((rc = krylov_solve(h, tolref, prm, x, res, true))) return rc;
+        if ((rc = krylov_solve(h, tolref, prm, x, res, pi))) return rc;
     }
     PCF_CUDA_TRY(cudaEventRecord(h->ev[3], h->stream));
     return PCF_OK;
@@ -3157,18 +3364,21 @@ int pcf_solve(pcf_handle *h, const double *rhs, const double *rho, const double 
         PCF_CUDA_TRY(cudaEventRecord(h->slab_ev[sl], h->copy_stream));
         PCF_CUDA_TRY(cudaStreamWaitEvent(h->stream, h->slab_ev[sl], 0));
         if (sl == 0) PCF_CUDA_TRY(cudaEventRecord(h->ev[1], h->stream));
-        if ((rc = assemble_chunks(h, dt, rayleigh_factor, prm->damp_horizontal_wind_on_rhs, c0, c1))) break;
+        if ((rc = assemble_chunks(h, dt, rayleigh_factor, prm->damp_horizontal_wind_on_rhs, c0, c1,
+                                  spectral_solve(h, prm))))
+            break;
     }
     PCF_CUDA_TRY(cudaMemcpyAsync(h->b64, rhs, sizeof(double) * h->d.n, cudaMemcpyHostToDevice, h->copy_stream));
     PCF_CUDA_TRY(cudaEventRecord(h->ev[7], h->copy_stream));
     const double *x = nullptr;
-    if (!rc) rc = solve_common(h, dt, rayleigh_factor, tolref, prm, res, &x, h->ev[7], true);
+    bool pi = false;
+    if (!rc) rc = solve_common(h, dt, rayleigh_factor, tolref, prm, res, &x, &pi, h->ev[7], true);
     if (rc) {
         cudaStreamWaitEvent(h->stream, h->ev[7], 0);  // no later call may meet the copy in flight
         return rc;
     }
     if (!res->errflag) {
-        k_unscale<<<vec_grid(h->d.n), 256, 0, h->stream>>>(x, h->pbar, h->rhobar, 1.0 / dt, h->d.nx, h->d.ny,
+        k_unscale<<<vec_grid(h->d.n), 256, 0, h->stream>>>(x, pi, h->pbar, h->rhobar, 1.0 / dt, h->d.nx, h->d.ny,
                                                            h->d.nz, h->dims.nbx, h->dims.nby, h->dims.nbz, h->nxx,
                                                            h->nyy, h->w64, 0, 0, 0, h->d.nx, h->d.ny);
         PCF_CUDA_TRY(cudaGetLastError());
@@ -3209,10 +3419,11 @@ int pcf_solve_device(pcf_handle *h, const double *d_rhs, const double *d_rho, co
     if (d_p) PCF_CUDA_TRY(cudaMemcpyAsync(h->p, d_p, hb, cudaMemcpyDeviceToDevice, h->stream));
     PCF_CUDA_TRY(cudaMemcpyAsync(h->b64, d_rhs, sizeof(double) * h->d.n, cudaMemcpyDeviceToDevice, h->stream));
     const double *x = nullptr;
-    int rc = solve_common(h, dt, rayleigh_factor, tolref, prm, res, &x);
+    bool pi = false;
+    int rc = solve_common(h, dt, rayleigh_factor, tolref, prm, res, &x, &pi);
     if (rc) return rc;
     if (!res->errflag) {
-        k_unscale<<<vec_grid(h->d.n), 256, 0, h->stream>>>(x, h->pbar, h->rhobar, 1.0 / dt, h->d.nx, h->d.ny,
+        k_unscale<<<vec_grid(h->d.n), 256, 0, h->stream>>>(x, pi, h->pbar, h->rhobar, 1.0 / dt, h->d.nx, h->d.ny,
                                                            h->d.nz, h->dims.nbx, h->dims.nby, h->dims.nbz, h->nxx,
                                                            h->nyy, d_dpip, h->dims.nbx, h->dims.nby, h->dims.nbz,
                                                            h->nxx, h->nyy);
@@ -3346,11 +3557,12 @@ struct pcf_ensemble {
     long long graph_launches = 0;
     long long launches = 0;
     bool key_valid = false;
-    bool use_sp = false, key_sp = false;  // spectral preconditioner: this solve's, the captured graph's
+    // spectral preconditioner and flux-form operator: this solve's, the captured graph's
+    bool use_sp = false, use_fx = false, key_sp = false, key_fx = false;
     int key_ci = 0, key_precond = 0, key_pc_iters = 0, key_mg = 0, key_mg_ci = 0, key_mg_min = 0, key_maxit = 0;
     double key_dtau = 0, key_mg_dtau = 0;
     KrylovScalars *h_status = nullptr;  // pinned, 2 slots x members
-    double *h_norm = nullptr;           // pinned, members
+    double *h_norm = nullptr;           // pinned, members; then as many words for k_flux_build's findings
     // the whole solve as one graph launch: a conditional WHILE node around
     // the batch, whose last kernel decides on the device whether to go on
     cudaGraphExec_t loop_exec = nullptr;
@@ -3379,6 +3591,7 @@ static LoopCfg ensemble_loop_cfg(const pcf_ensemble *e, pcf_handle *h, const pcf
     c.flex = 1;
     c.reliable = 1;
     c.sp = e->use_sp ? 1 : 0;
+    c.fx = e->use_fx ? 1 : 0;
     c.mg = prm->multigrid && !c.sp ? 1 : 0;
     if (c.mg) c.deta = h->mg->lv[0].deta;
     return c;
@@ -3505,6 +3718,7 @@ static int ensemble_capture(pcf_ensemble *e, const pcf_params *prm, int ci) {
     e->key_mg_dtau = prm->mg_dtau;
     e->key_maxit = prm->poisson_iterations;
     e->key_sp = e->use_sp;
+    e->key_fx = e->use_fx;
     return ensemble_capture_loop(e, prm, ci, (prm->poisson_iterations + ci - 1) / ci);
 }
 
@@ -3551,7 +3765,7 @@ int pcf_ensemble_create(pcf_ensemble **out, pcf_handle *const *members, int coun
     for (cudaEvent_t &x : e->join)
         if (cudaEventCreateWithFlags(&x, cudaEventDisableTiming) != cudaSuccess) return fail(PCF_ECUDA);
     if (cudaMallocHost((void **)&e->h_status, 2 * sizeof(KrylovScalars) * count) != cudaSuccess) return fail(PCF_ENOMEM);
-    if (cudaMallocHost((void **)&e->h_norm, sizeof(double) * count) != cudaSuccess) return fail(PCF_ENOMEM);
+    if (cudaMallocHost((void **)&e->h_norm, 2 * sizeof(double) * count) != cudaSuccess) return fail(PCF_ENOMEM);
     *out = e;
     return PCF_OK;
 }
@@ -3597,7 +3811,8 @@ int pcf_ensemble_solve_device(pcf_ensemble *e, const double *const *d_rhs, const
         if (d_p && d_p[q]) PCF_CUDA_TRY(cudaMemcpyAsync(h->p, d_p[q], hb, cudaMemcpyDeviceToDevice, h->stream));
         PCF_CUDA_TRY(cudaMemcpyAsync(h->b64, d_rhs[q], sizeof(double) * h->d.n, cudaMemcpyDeviceToDevice, h->stream));
         PCF_CUDA_TRY(cudaEventRecord(h->ev[1], h->stream));
-        if ((rc = assemble_device(h, dt[q], rayleigh_factor[q], prm->damp_horizontal_wind_on_rhs))) return rc;
+        if ((rc = assemble_device(h, dt[q], rayleigh_factor[q], prm->damp_horizontal_wind_on_rhs, e->use_sp)))
+            return rc;
         if (prm->preconditioner && !prm->multigrid && (rc = ensure_factors(h, deta_of(h, prm->dtau)))) return rc;
         if (e->use_sp ? (rc = spectral_prepare(h)) : prm->multigrid ? (rc = mg_prepare(h, prm, true)) : 0) return rc;
         if (prm->autotune && (rc = autotune_handle(h, prm))) return rc;
@@ -3609,13 +3824,29 @@ int pcf_ensemble_solve_device(pcf_ensemble *e, const double *const *d_rhs, const
         h->launches += 1;
         PCF_CUDA_TRY(cudaGetLastError());
         PCF_CUDA_TRY(cudaMemcpyAsync(e->h_norm + q, h->dot_out, sizeof(double), cudaMemcpyDeviceToHost, h->stream));
+        if (e->use_sp)
+            PCF_CUDA_TRY(cudaMemcpyAsync(e->h_norm + n + q, h->ticket + 2, sizeof(unsigned), cudaMemcpyDeviceToHost,
+                                         h->stream));
     }
     for (int q = 0; q < n; ++q) PCF_CUDA_TRY(cudaStreamSynchronize(e->m[q]->stream));
+    e->use_fx = e->use_sp;
+    for (int q = 0; q < n && e->use_fx; ++q) {
+        unsigned uneven;
+        std::memcpy(&uneven, e->h_norm + n + q, sizeof(uneven));
+        e->use_fx = uneven == 0;
+    }
+    if (e->use_sp && !e->use_fx) {
+        // halo columns that are not the periodic image: the planes tell them apart
+        for (int q = 0; q < n; ++q)
+            if ((rc = ensure_planes(e->m[q])) || (rc = spectral_prepare(e->m[q]))) return rc;
+        for (int q = 0; q < n; ++q) PCF_CUDA_TRY(cudaStreamSynchronize(e->m[q]->stream));
+    }
     // the iteration graph, captured with every stream idle
     if (!e->exec || !e->key_valid || e->key_ci != ci || e->key_precond != prm->preconditioner ||
         e->key_pc_iters != prm->preconditioner_iterations || e->key_dtau != prm->dtau || e->key_mg != prm->multigrid ||
         e->key_mg_ci != prm->mg_coarse_iterations || e->key_mg_min != prm->mg_min_columns ||
-        e->key_mg_dtau != prm->mg_dtau || e->key_maxit != prm->poisson_iterations || e->key_sp != e->use_sp) {
+        e->key_mg_dtau != prm->mg_dtau || e->key_maxit != prm->poisson_iterations || e->key_sp != e->use_sp ||
+        e->key_fx != e->use_fx) {
         if ((rc = ensemble_capture(e, prm, ci))) return rc;
     }
     std::vector<double> bnorm(n), tol(n);
@@ -3701,6 +3932,7 @@ int pcf_ensemble_solve_device(pcf_ensemble *e, const double *const *d_rhs, const
         pcf_handle *h = e->m[q];
         PCF_CUDA_TRY(cudaStreamWaitEvent(h->stream, e->done, 0));
         const double *x = h->x64;
+        bool pi = e->use_fx;
         if (active[q]) {
             const LoopCfg c = ensemble_loop_cfg(e, h, prm);
             const Work<float> w = work32_pi(h);
@@ -3709,7 +3941,7 @@ int pcf_ensemble_solve_device(pcf_ensemble *e, const double *const *d_rhs, const
             if ((rc = run_finish<float>(h, w, c, false, 0, &xe, &ro))) return rc;
             res[q].niter = ro.iters;
             res[q].nrefine = ro.nupdates;
-            reliable_bytes(h, ro.nupdates);
+            reliable_bytes(h, ro.nupdates, e->use_fx ? flux_words(h) : 28.0);
             res[q].status = ro.status;
             res[q].residual = res[q].true_residual = ro.nupdates > 0 ? ro.res : 1.0;
             const bool converged = ro.converged || (e->use_sp && ro.status == PCF_OK && res[q].residual <= tol[q]);
@@ -3721,6 +3953,7 @@ int pcf_ensemble_solve_device(pcf_ensemble *e, const double *const *d_rhs, const
                 pcf_params again = *prm;
                 if (e->use_sp) again.poisson_iterations = std::max(1, maxit - ro.iters);
                 if ((rc = krylov_solve(h, tolref[q], &again, &x, &r2))) return rc;
+                pi = false;
                 r2.niter += res[q].niter;
                 r2.nrefine += res[q].nrefine;
                 res[q] = r2;
@@ -3730,7 +3963,7 @@ int pcf_ensemble_solve_device(pcf_ensemble *e, const double *const *d_rhs, const
         }
         PCF_CUDA_TRY(cudaEventRecord(h->ev[3], h->stream));
         if (!res[q].errflag) {
-            k_unscale<<<vec_grid(h->d.n), 256, 0, h->stream>>>(x, h->pbar, h->rhobar, 1.0 / dt[q], h->d.nx, h->d.ny,
+            k_unscale<<<vec_grid(h->d.n), 256, 0, h->stream>>>(x, pi, h->pbar, h->rhobar, 1.0 / dt[q], h->d.nx, h->d.ny,
                                                                h->d.nz, h->dims.nbx, h->dims.nby, h->dims.nbz, h->nxx,
                                                                h->nyy, d_dpip[q], h->dims.nbx, h->dims.nby,
                                                                h->dims.nbz, h->nxx, h->nyy);
