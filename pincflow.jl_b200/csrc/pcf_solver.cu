@@ -1370,7 +1370,10 @@ static int spectral_create(pcf_handle *h) {
     s->gy = dim3((unsigned)((a.npair + ly - 1) / ly), (unsigned)nz);
     s->smx = 2 * sizeof(float2) * (size_t)fpad_size(lx * nx);
     s->smy = 2 * sizeof(float2) * (size_t)fpad_size(ly * ny);
-    s->ch = nz <= 128 ? 4 : nz <= 256 ? 8 : 16;
+    // levels per run: 4 where the columns are short (all of them in flight at
+    // once), 8 from there, so that a block's chain over the runs stays short and
+    // two blocks fit an SM (256x256x128: 44 us with 4, 27 with 8), 16 beyond 256
+    s->ch = nz <= 32 ? 4 : nz <= 256 ? 8 : 16;
     s->gz = dim3((unsigned)((a.npair + 31) / 32), (unsigned)ny);
     s->bz = dim3(32, (unsigned)((nz + s->ch - 1) / s->ch));
     a.lines = lx;  // the y kernels' count is set at their launches
