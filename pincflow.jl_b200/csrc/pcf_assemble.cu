@@ -33,7 +33,7 @@ namespace pcf {
 struct AssembleArgs {
     int nx, ny, nz, nxx, nyy, nbx, nby, nbz;
     int z_size, ko, model, damp_h;
-    int kc0;  // first z-chunk (of AKC levels) of the launch
+    int l0, l1, kpb;  // levels [l0, l1) of the launch, kpb of them per block
     double dx, dy, dz, dt, rf;
     double rdx, rdy, rdz;  // 1 / dx, 1 / dy, 1 / dz
     double gamma, kappa, rsp, pref;
@@ -64,8 +64,8 @@ __device__ __forceinline__ int level_case(int kg, int nbz, int z_size) {
 }
 
 // ---- staging -------------------------------------------------------------
-// A block assembles a tile of AX x AY columns over AKC levels, marching up in
-// z.  Every input it reads lies within one column in x and y and two levels
+// A block assembles a tile of AX x AY columns over at most AKC levels, marching up
+// in z.  Every input it reads lies within one column in x and y and two levels
 // in z of the cell, so each level of each input field is copied once per block
 // into a shared-memory ring (cp.async, 8 bytes per element) and every cell
 // reads its neighbourhood from there.  The copy of level k + 2 (k + 3 for the
@@ -147,8 +147,8 @@ __global__ void __launch_bounds__(AX * AY, 3) k_assemble(AssembleArgs a) {
     extern __shared__ double asm_sm[];
     const int tid = threadIdx.x + AX * threadIdx.y;
     const int tx = threadIdx.x, ty = threadIdx.y;
-    const int i0 = blockIdx.x * AX, j0 = blockIdx.y * AY, k0 = (blockIdx.z + a.kc0) * AKC;
-    const int k1 = min(k0 + AKC, a.nz);
+    const int i0 = blockIdx.x * AX, j0 = blockIdx.y * AY, k0 = a.l0 + blockIdx.z * a.kpb;
+    const int k1 = min(k0 + a.kpb, a.l1);
     const int ii = i0 + tx, jj = j0 + ty;
     const bool live = ii < a.nx && jj < a.ny;
     const long long n = (long long)a.nx * a.ny * a.nz;
@@ -494,9 +494,15 @@ int pcf_launch_assemble(pcf_handle *h, double dt, double rf, int damp_h, int c0,
     const int nchunks = (h->d.nz + pcf::AKC - 1) / pcf::AKC;
     if (c1 < 0 || c1 > nchunks) c1 = nchunks;
     if (c0 < 0 || c0 >= c1) return PCF_OK;
-    a.kc0 = c0;
-    const dim3 grid((unsigned)((h->d.nx + pcf::AX - 1) / pcf::AX), (unsigned)((h->d.ny + pcf::AY - 1) / pcf::AY),
-                    (unsigned)(c1 - c0));
+    a.l0 = c0 * pcf::AKC;
+    a.l1 = c1 * pcf::AKC < h->d.nz ? c1 * pcf::AKC : h->d.nz;
+    const int gx = (h->d.nx + pcf::AX - 1) / pcf::AX, gy = (h->d.ny + pcf::AY - 1) / pcf::AY;
+    // fewer levels per block where AKC would leave less than two blocks per SM:
+    // a block takes about 6 us per level, whatever the grid (64x64x32: 64 blocks
+    // of 16 levels, 107 us)
+    a.kpb = pcf::AKC;
+    while (a.kpb > 2 && (long long)gx * gy * ((a.l1 - a.l0 + a.kpb - 1) / a.kpb) < 2 * 148) a.kpb /= 2;
+    const dim3 grid((unsigned)gx, (unsigned)gy, (unsigned)((a.l1 - a.l0 + a.kpb - 1) / a.kpb));
     pcf::k_assemble<<<grid, dim3(pcf::AX, pcf::AY), pcf::ASM_SMEM, h->stream>>>(a);
     PCF_CUDA_TRY(cudaGetLastError());
     h->fac_deta = __builtin_nan("");
