@@ -78,32 +78,55 @@ __device__ double grad_h(const CorrectArgs &a, const double *P, const Ix &at, in
     return a.kappainv * a.mainv2 * pe / rhoe * ((P[n] - P[c]) * rh + mete * dz * 0.5 * a.rdz);
 }
 
-// compute_pressure_gradient of the field P for W at (i, j, k+1/2)
-// (compute_pressure_gradient.jl:212-297) for the point c at level k.  The
-// halo (nbx, nby >= 1, nbz >= 2) keeps the levels k0-1 and k1+1 in bounds.
-__device__ __forceinline__ double grad_w_at(const CorrectArgs &a, const double *P, long long c, long long sy,
-                                            long long sz) {
+// What the W and RhoP kernels take from the face above a cell: Jacobian
+// weights of the two levels, the reciprocal of the face density and the
+// pressure gradient there (compute_pressure_gradient of the field P for W,
+// compute_pressure_gradient.jl:212-297).  The halo (nbx, nby >= 1, nbz >= 2)
+// keeps the levels k0-1 and k1+1 in bounds.
+struct Face {
+    double th, tu;  // weights of the level below and above: (J_u, J_c) / (J_c + J_u)
+    double rj;      // 1 / (J_c + J_u)
+    double rrho;    // 1 / (face density)
+    double grad;    // pressure gradient
+};
+__device__ __forceinline__ Face face_above(const CorrectArgs &a, const double *P, long long c, long long sy,
+                                           long long sz, double jc, double ju, double rc, double ru) {
+    Face f;
     const long long u = c + sz;
+    f.rj = 1.0 / (jc + ju);
+    f.th = ju * f.rj;
+    f.tu = jc * f.rj;
+    f.rrho = 1.0 / (f.th * rc + f.tu * ru);
     const double *J = a.jac;
-    const double jk = J[c], jk1 = J[u], rj = 1.0 / (jk + jk1);
-    const double rhoe = (jk1 * a.rho[c] + jk * a.rho[u]) * rj + (jk1 * a.rhobar[c] + jk * a.rhobar[u]) * rj;
-    const double pe = (jk1 * a.pbar[c] + jk * a.pbar[u]) * rj;
-    const double m13 = (jk1 * a.met13[c] + jk * a.met13[u]) * rj;
-    const double m23 = (jk1 * a.met23[c] + jk * a.met23[u]) * rj;
-    const double m33 = (jk1 * a.met33[c] + jk * a.met33[u]) * rj;
-    auto edge = [&](long long q) {  // Jacobian-weighted P at the w-level of column q
-        return (J[q + sz] * P[q] + J[q] * P[q + sz]) / (J[q] + J[q + sz]);
+    // the difference of the Jacobian-weighted P of two columns at the face, over one denominator
+    auto across = [&](long long h, long long l) {
+        const double h0 = J[h], h1 = J[h + sz], l0 = J[l], l1 = J[l + sz], dh = h0 + h1, dl = l0 + l1;
+        return ((h1 * P[h] + h0 * P[h + sz]) * dl - (l1 * P[l] + l0 * P[l + sz]) * dh) / (dh * dl);
     };
-    const double pr = edge(c + 1), pl = edge(c - 1), pf = edge(c + sy), pb = edge(c - sy);
-    return a.kappainv * a.mainv2 * pe / rhoe *
-           (m13 * (pr - pl) * 0.5 * a.rdx + m23 * (pf - pb) * 0.5 * a.rdy + m33 * (P[u] - P[c]) * a.rdz);
+    const double m13 = f.th * a.met13[c] + f.tu * a.met13[u], m23 = f.th * a.met23[c] + f.tu * a.met23[u];
+    const double m33 = f.th * a.met33[c] + f.tu * a.met33[u], pe = f.th * a.pbar[c] + f.tu * a.pbar[u];
+    f.grad = a.kappainv * a.mainv2 * pe * f.rrho *
+             (m13 * across(c + 1, c - 1) * 0.5 * a.rdx + m23 * across(c + sy, c - sy) * 0.5 * a.rdy +
+              m33 * (P[u] - P[c]) * a.rdz);
+    return f;
 }
 
-// The pointwise kernels below are chains of dependent FP64 divisions and
-// products: they run at as many resident warps as 64 registers a thread
-// allow (4 blocks of 256 per SM), which hides those latencies better than
-// fewer threads with more loads in flight each.
+// The pointwise kernels are chains of dependent FP64 divisions (about 20
+// instructions each) and products: they run at as many resident warps as 64
+// registers a thread allow (4 blocks of 256 per SM), which hides those
+// latencies better than fewer threads with more loads in flight each (marching
+// up a column with the lower face carried took 128 registers and 1.4 times as
+// long).  So what has one denominator is put over it: a cell of the W and RhoP
+// predictors takes 16-17 divisions each instead of 35-40 (192x160x96,
+// Compressible with waves and damping: the predictor 788 -> 678 us).
 #define PCF_POINTWISE_BOUNDS __launch_bounds__(256, 4)
+
+// total density, and the buoyancy factor's numerator (over the total density)
+__device__ __forceinline__ double total_rho(const CorrectArgs &a, long long c) { return a.rho[c] + a.rhobar[c]; }
+template <bool COMP>
+__device__ __forceinline__ double buoyancy(const CorrectArgs &a, long long c) {
+    return COMP ? a.pbar[c] / a.thetabar[c] : a.rhobar[c];
+}
 
 // U and V corrections (correct!.jl:177-245) with corx, cory: thread (x, y, k)
 // over (nx + 1) x (ny + 1) x nz staggered positions; x = 0 is the face i0 - 1/2.
@@ -155,39 +178,28 @@ __global__ void PCF_POINTWISE_BOUNDS k_correct_w_rhop_pip(CorrectArgs a) {
     const bool interior = x >= 1 && x <= a.nx && y >= 1 && y <= a.ny && z >= 1 && z <= a.nz;
     if (!interior) return;
     const double *J = a.jac;
-    const long long u = c + sz, l = c - 1, b = c - sy;
+    const long long u = c + sz, d = c - sz;
     const bool top = k == a.nbz + a.nz - 1, bot = k == a.nbz;
-    const double gu = top ? 0.0 : grad_w_at(a, a.dpip, c, sy, sz);
+    auto cross = [&](long long q) {
+        return a.met13[q] * (a.corx[q] + a.corx[q - 1]) + a.met23[q] * (a.cory[q] + a.cory[q - sy]);
+    };
+    const double jc = J[c], rc = total_rho(a, c), xc = cross(c), nc = buoyancy<COMP>(a, c);
+    double above = 0.0;
     if (!top) {  // W at k + 1/2 for k in k0 .. k1-1
-        const double rj = 1.0 / (J[c] + J[u]);
-        const double factor = 1.0 + a.dt * (J[u] * a.betar[c] + J[c] * a.betar[u]) * rj * a.rf;
-        const double n2e = (J[u] * a.n2[c] + J[c] * a.n2[u]) * rj;
-        double jp = 1.0, fw;
-        const double den = J[u] * (a.rho[c] + a.rhobar[c]) + J[c] * (a.rho[u] + a.rhobar[u]);
-        if (COMP) {
-            jp = J[c] * J[u] * (a.p[c] + a.p[u]) * rj;
-            fw = (J[u] * a.pbar[c] / a.thetabar[c] + J[c] * a.pbar[u] / a.thetabar[u]) / den;
-        } else {
-            fw = (J[u] * a.rhobar[c] + J[c] * a.rhobar[u]) / den;
-        }
-        const double inv = 1.0 / (factor + fw * n2e * dt2);
-        const double cross = (J[u] * (a.met13[c] * (a.corx[c] + a.corx[l]) + a.met23[c] * (a.cory[c] + a.cory[b])) +
-                              J[c] * (a.met13[u] * (a.corx[u] + a.corx[l + sz]) +
-                                      a.met23[u] * (a.cory[u] + a.cory[b + sz]))) * rj;
-        a.w[c] += -a.dt * inv * jp * gu - inv * fw * n2e * dt2 * jp * 0.5 * cross;
+        const double ju = J[u], ru = total_rho(a, u);
+        const Face f = face_above(a, a.dpip, c, sy, sz, jc, ju, rc, ru);
+        above = f.grad;
+        const double factor = 1.0 + a.dt * (f.th * a.betar[c] + f.tu * a.betar[u]) * a.rf;
+        const double n2e = f.th * a.n2[c] + f.tu * a.n2[u];
+        const double jp = COMP ? jc * ju * (a.p[c] + a.p[u]) * f.rj : 1.0;
+        // buoyancy factor b / den
+        const double den = ju * rc + jc * ru, b = (ju * nc + jc * buoyancy<COMP>(a, u)) * n2e * dt2;
+        a.w[c] -= jp * (a.dt * above * den + b * 0.5 * (f.th * xc + f.tu * cross(u))) / (factor * den + b);
     }
-    // rho'
-    const double gl = bot ? 0.0 : grad_w_at(a, a.dpip, c - sz, sy, sz);
-    const double gradient = 0.5 * (gl + gu);
-    const double factor = 1.0 + a.dt * a.betar[c] * a.rf;
-    const double fb = COMP ? a.pbar[c] / a.thetabar[c] / (a.rho[c] + a.rhobar[c])
-                           : a.rhobar[c] / (a.rho[c] + a.rhobar[c]);
-    const double n2c = a.n2[c];
-    const double db = -1.0 / (factor + fb * n2c * dt2) *
-                      (-fb * n2c * dt2 * J[c] * gradient +
-                       fb * n2c * a.dt * J[c] * factor * 0.5 *
-                           (a.met13[c] * (a.corx[c] + a.corx[l]) + a.met23[c] * (a.cory[c] + a.cory[b])));
-    a.rhop[c] -= (a.rho[c] + a.rhobar[c]) / a.g_ndim * db;
+    const double below = bot ? 0.0 : face_above(a, a.dpip, d, sy, sz, J[d], jc, total_rho(a, d), rc).grad;
+    const double factor = 1.0 + a.dt * a.betar[c] * a.rf, b = nc * a.n2[c];
+    const double db = -b * jc * (-dt2 * 0.5 * (below + above) + a.dt * factor * 0.5 * xc) / (factor * rc + b * dt2);
+    a.rhop[c] -= rc / a.g_ndim * db;
 }
 
 // ------------------------------------------------------------ predictor --
@@ -324,7 +336,8 @@ __global__ void PCF_POINTWISE_BOUNDS k_predict_uv(CorrectArgs a) {
             double factor = 1.0;
             if (a.damp_h) factor += a.dt * 0.5 * (a.betar[c] + a.betar[n]) * a.rf;
             const double jp = wind_factor_u(a, c, 1);
-            a.u[c] = 1.0 / factor * (a.u[c] + a.dt * (-gradient + force / rhoe) * jp);
+            const double un = a.u[c] + a.dt * ((a.dudt ? force / rhoe : 0.0) - gradient) * jp;
+            a.u[c] = a.damp_h ? un / factor : un;
         }
         if (x >= 1) {  // V at j + 1/2 for j in j0-1 .. j1
             const long long n = c + at.sy;
@@ -335,7 +348,8 @@ __global__ void PCF_POINTWISE_BOUNDS k_predict_uv(CorrectArgs a) {
             double factor = 1.0;
             if (a.damp_h) factor += a.dt * 0.5 * (a.betar[c] + a.betar[n]) * a.rf;
             const double jp = wind_factor_u(a, c, at.sy);
-            a.v[c] = 1.0 / factor * (a.v[c] + a.dt * (-gradient + force / rhoe) * jp);
+            const double vn = a.v[c] + a.dt * ((a.dvdt ? force / rhoe : 0.0) - gradient) * jp;
+            a.v[c] = a.damp_h ? vn / factor : vn;
         }
     }
 }
@@ -347,27 +361,24 @@ template <bool COMP>
 __device__ __forceinline__ double jp_uv(const CorrectArgs &a, long long c, long long o) {
     return COMP ? (a.jac[c] * a.p[c] + a.jac[c + o] * a.p[c + o]) / 2 : 1.0;
 }
-template <bool COMP>
-__device__ __forceinline__ double jp_w(const CorrectArgs &a, long long c, long long sz) {
-    if (!COMP) return 1.0;
-    const double jk = a.jac[c], jk1 = a.jac[c + sz];
-    return jk * jk1 * (a.p[c] + a.p[c + sz]) / (jk + jk1);
-}
-
-// compute_volume_force(state, i, j, k, W()) (compute_volume_force.jl:185-206)
-__device__ __forceinline__ double force_w(const CorrectArgs &a, long long c, long long sz) {
-    if (!a.dudt) return 0.0;
-    const double *J = a.jac;
-    const long long u = c + sz;
-    return (J[u] * (a.met13[c] * a.dudt[c] + a.met23[c] * a.dvdt[c]) +
-            J[c] * (a.met13[u] * a.dudt[u] + a.met23[u] * a.dvdt[u])) /
-           (J[c] + J[u]);
-}
-
 // x / y, or x when y is the non-compressible wind factor 1 (exact either way)
 template <bool COMP>
 __device__ __forceinline__ double over(double x, double y) {
     return COMP ? x / y : x;
+}
+
+// met13 u + met23 v with the winds averaged to the cell (divided by the
+// compressible wind factors): the terrain-following part of the vertical wind
+template <bool COMP>
+__device__ __forceinline__ double wind_cross(const CorrectArgs &a, long long c, long long sy) {
+    const long long l = c - 1, b = c - sy;
+    return a.met13[c] * 0.5 * (over<COMP>(a.u[c], jp_uv<COMP>(a, c, 1)) + over<COMP>(a.u[l], jp_uv<COMP>(a, l, 1))) +
+           a.met23[c] * 0.5 * (over<COMP>(a.v[c], jp_uv<COMP>(a, c, sy)) + over<COMP>(a.v[b], jp_uv<COMP>(a, b, sy)));
+}
+
+// met13 dudt + met23 dvdt (compute_volume_force.jl:185-206 before its face mean)
+__device__ __forceinline__ double wave_cross(const CorrectArgs &a, long long c) {
+    return a.dudt ? a.met13[c] * a.dudt[c] + a.met23[c] * a.dvdt[c] : 0.0;
 }
 
 // update!(W, RHS(), Implicit()) (update!.jl:1248-1336) for k in k0 .. k1-1,
@@ -379,37 +390,20 @@ __global__ void PCF_POINTWISE_BOUNDS k_predict_w(CorrectArgs a) {
     const double *J = a.jac;
     const int x = blockIdx.x * blockDim.x + threadIdx.x, y = blockIdx.y * blockDim.y + threadIdx.y, z = blockIdx.z;
     if (x >= a.nx || y >= a.ny) return;
-    const long long c = (a.nbx + x) + sy * (a.nby + y) + sz * (a.nbz + z), u = c + sz, l = c - 1, b = c - sy;
-    const double rj = J[c] + J[u];
-    double rhoc = a.rho[c];
-    double rhou = a.rho[u];
-    double rhoedgeu = (J[u] * a.rho[c] + J[c] * a.rho[u]) / rj;
-    rhoc += a.rhobar[c];
-    rhou += a.rhobar[u];
-    rhoedgeu += (J[u] * a.rhobar[c] + J[c] * a.rhobar[u]) / rj;
-    const double gradient = grad_w_at(a, a.pip, c, sy, sz);
-    const double force = force_w(a, c, sz);
-    const double n2edgeu = (J[u] * a.n2[c] + J[c] * a.n2[u]) / rj;
-    double factor = 1.0;
-    factor += a.dt * (J[u] * a.betar[c] + J[c] * a.betar[u]) / rj * a.rf;
-    const double bb = -a.g_ndim * (J[u] * a.rhop[c] / rhoc / J[c] + J[c] * a.rhop[u] / rhou / J[u]) / rj;
-    const double uc = 0.5 * (over<COMP>(a.u[c], jp_uv<COMP>(a, c, 1)) + over<COMP>(a.u[l], jp_uv<COMP>(a, l, 1)));
-    const double uu = 0.5 * (over<COMP>(a.u[u], jp_uv<COMP>(a, u, 1)) +
-                             over<COMP>(a.u[l + sz], jp_uv<COMP>(a, l + sz, 1)));
-    const double vc = 0.5 * (over<COMP>(a.v[c], jp_uv<COMP>(a, c, sy)) + over<COMP>(a.v[b], jp_uv<COMP>(a, b, sy)));
-    const double vu = 0.5 * (over<COMP>(a.v[u], jp_uv<COMP>(a, u, sy)) +
-                             over<COMP>(a.v[b + sz], jp_uv<COMP>(a, b + sz, sy)));
-    const double jpedgeu = jp_w<COMP>(a, c, sz);
-    double fw;
-    const double den = J[u] * (a.rho[c] + a.rhobar[c]) + J[c] * (a.rho[u] + a.rhobar[u]);
-    if (COMP)
-        fw = (J[u] * a.pbar[c] / a.thetabar[c] + J[c] * a.pbar[u] / a.thetabar[u]) / den;
-    else
-        fw = (J[u] * a.rhobar[c] + J[c] * a.rhobar[u]) / den;
-    a.w[c] = 1.0 / (factor + fw * n2edgeu * dt2) *
-             (a.w[c] - a.dt * gradient * jpedgeu + a.dt * bb * jpedgeu + a.dt * force / rhoedgeu * jpedgeu +
-              jpedgeu * fw * n2edgeu * dt2 *
-                  (J[u] * (a.met13[c] * uc + a.met23[c] * vc) + J[c] * (a.met13[u] * uu + a.met23[u] * vu)) / rj);
+    const long long c = (a.nbx + x) + sy * (a.nby + y) + sz * (a.nbz + z), u = c + sz;
+    if (!PCF_IN(u, sz * (a.nz + 2 * a.nbz), 504)) return;
+    const double jc = J[c], ju = J[u], rc = total_rho(a, c), ru = total_rho(a, u);
+    const Face f = face_above(a, a.pip, c, sy, sz, jc, ju, rc, ru);
+    const double factor = 1.0 + a.dt * (f.th * a.betar[c] + f.tu * a.betar[u]) * a.rf;
+    const double n2e = f.th * a.n2[c] + f.tu * a.n2[u];
+    const double bb = -a.g_ndim * (ju * a.rhop[c] / (rc * jc) + jc * a.rhop[u] / (ru * ju)) * f.rj;
+    const double force = (f.th * wave_cross(a, c) + f.tu * wave_cross(a, u)) * f.rrho;
+    const double jp = COMP ? jc * ju * (a.p[c] + a.p[u]) * f.rj : 1.0;
+    // buoyancy factor b / den
+    const double den = ju * rc + jc * ru, b = (ju * buoyancy<COMP>(a, c) + jc * buoyancy<COMP>(a, u)) * n2e * dt2;
+    a.w[c] = (den * (a.w[c] + a.dt * jp * (bb - f.grad + force)) +
+              jp * b * (f.th * wind_cross<COMP>(a, c, sy) + f.tu * wind_cross<COMP>(a, u, sy))) /
+             (factor * den + b);
 }
 
 // update!(RhoP, RHS(), Implicit()) (update!.jl:632-728) on the interior,
@@ -421,33 +415,30 @@ __global__ void PCF_POINTWISE_BOUNDS k_predict_rhop(CorrectArgs a) {
     const double *J = a.jac;
     const int x = blockIdx.x * blockDim.x + threadIdx.x, y = blockIdx.y * blockDim.y + threadIdx.y, z = blockIdx.z;
     if (x >= a.nx || y >= a.ny) return;
-    const long long c = (a.nbx + x) + sy * (a.nby + y) + sz * (a.nbz + z), u = c + sz, d = c - sz, l = c - 1,
-                    b = c - sy;
-    const double rhoc = a.rho[c] + a.rhobar[c];
-    double rhoedgeu = (J[u] * a.rho[c] + J[c] * a.rho[u]) / (J[c] + J[u]);
-    rhoedgeu += (J[u] * a.rhobar[c] + J[c] * a.rhobar[u]) / (J[c] + J[u]);
-    double rhoedged = (J[d] * a.rho[c] + J[c] * a.rho[d]) / (J[c] + J[d]);
-    rhoedged += (J[d] * a.rhobar[c] + J[c] * a.rhobar[d]) / (J[c] + J[d]);
-    const double wv = 0.5 * (over<COMP>(a.wold[c], jp_w<COMP>(a, c, sz)) + over<COMP>(a.wold[d], jp_w<COMP>(a, d, sz)));
-    const bool bot = z == 0, top = z == a.nz - 1 && !bot;
-    const double lower_gradient = bot ? 0.0 : grad_w_at(a, a.pip, d, sy, sz);
-    const double lower_force = bot ? 0.0 : force_w(a, d, sz);
-    const double upper_gradient = top ? 0.0 : grad_w_at(a, a.pip, c, sy, sz);
-    const double upper_force = top ? 0.0 : force_w(a, c, sz);
-    const double gradient = 0.5 * (lower_gradient + upper_gradient);
-    const double force = 0.5 * (lower_force / rhoedged + upper_force / rhoedgeu) * rhoc;
-    double factor = 1.0;
-    factor += a.dt * a.betar[c] * a.rf;
-    double bb = -a.g_ndim * a.rhop[c] / (a.rho[c] + a.rhobar[c]);
-    const double fb = COMP ? a.pbar[c] / a.thetabar[c] / (a.rho[c] + a.rhobar[c])
-                           : a.rhobar[c] / (a.rho[c] + a.rhobar[c]);
-    const double n2c = a.n2[c], jc = J[c];
-    bb = 1.0 / (factor + fb * n2c * dt2) *
-         (-fb * n2c * a.dt * jc * (wv + a.dt * (-gradient + force / rhoc)) + factor * bb +
-          fb * n2c * a.dt * jc * factor * 0.5 *
-              (a.met13[c] * (over<COMP>(a.u[c], jp_uv<COMP>(a, c, 1)) + over<COMP>(a.u[l], jp_uv<COMP>(a, l, 1))) +
-               a.met23[c] * (over<COMP>(a.v[c], jp_uv<COMP>(a, c, sy)) + over<COMP>(a.v[b], jp_uv<COMP>(a, b, sy)))));
-    a.rhop[c] = -bb * (a.rho[c] + a.rhobar[c]) / a.g_ndim;
+    const long long c = (a.nbx + x) + sy * (a.nby + y) + sz * (a.nbz + z), u = c + sz, d = c - sz;
+    if (!PCF_IN(u, sz * (a.nz + 2 * a.nbz), 505)) return;
+    // the old vertical wind at the face above q, over the compressible wind factor
+    auto old_wind = [&](long long q, double jq, double jn) {
+        return COMP ? a.wold[q] * (jq + jn) / (jq * jn * (a.p[q] + a.p[q + sz])) : a.wold[q];
+    };
+    const double jc = J[c], ju = J[u], jd = J[d], rc = total_rho(a, c), fc = wave_cross(a, c);
+    const bool bot = z == 0, top = z == a.nz - 1;
+    double acc = 0.0;  // force minus gradient at the face above plus below (0 at the walls)
+    if (!top) {
+        const Face f = face_above(a, a.pip, c, sy, sz, jc, ju, rc, total_rho(a, u));
+        acc = (f.th * fc + f.tu * wave_cross(a, u)) * f.rrho - f.grad;
+    }
+    if (!bot) {
+        const Face f = face_above(a, a.pip, d, sy, sz, jd, jc, total_rho(a, d), rc);
+        acc += (f.th * wave_cross(a, d) + f.tu * fc) * f.rrho - f.grad;
+    }
+    const double wv = old_wind(c, jc, ju) + old_wind(d, jd, jc);
+    const double factor = 1.0 + a.dt * a.betar[c] * a.rf;
+    const double b = buoyancy<COMP>(a, c) * a.n2[c];  // buoyancy factor b / rc
+    const double bb = (-b * a.dt * jc * 0.5 * (wv + a.dt * acc) - factor * a.g_ndim * a.rhop[c] +
+                       b * a.dt * jc * factor * wind_cross<COMP>(a, c, sy)) /
+                      (factor * rc + b * dt2);
+    a.rhop[c] = -bb * rc / a.g_ndim;
 }
 
 }  // namespace pcf
