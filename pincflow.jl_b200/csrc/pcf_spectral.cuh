@@ -20,7 +20,10 @@
 // V-cycle: about 330 and 60 launches).  Whole solves, V-cycle -> spectral:
 // 64x64x32 3.95 -> 0.97 ms, 150x90x45 24.2 -> 1.46 (the V-cycle's coarsening
 // ends at 75x45), 128x128x64 9.29 -> 1.87, 256x256x128 30.0 -> 7.07,
-// 512x512x192 153 -> 37.4, 32 ensemble members 186 -> 65.
+// 512x512x192 153 -> 37.4, 32 ensemble members 186 -> 65 (with the
+// coefficient planes; in flux form, pcf_flux.cuh, less again).
+// At 512x512x192 the passes take 150-200 us where their traffic takes 62-154:
+// index arithmetic, shared-memory passes and barriers.
 //
 // Layout of the transformed field (spec): rows of nxs floats, one per (j, k),
 // holding npair complex values.  Pair i >= 1 of row j is the coefficient of
@@ -178,13 +181,15 @@ __device__ __forceinline__ void fft_stage(const FftPlan &P, int st, const float2
         float2 v[R];
 #pragma unroll
         for (int q = 0; q < R; ++q) v[q] = in[fpad(XMAJOR ? l * n + j + q * m : (j + q * m) * lines + l)];
-        if (k) {
+        if (Ns > 1) {
+            // the twiddles are powers of one table entry: six loads fewer per butterfly
+            float2 w[R];
+            w[1] = __ldg(P.tw + k * step);
+            if (INV) w[1].y = -w[1].y;
 #pragma unroll
-            for (int q = 1; q < R; ++q) {
-                float2 w = __ldg(P.tw + q * k * step);
-                if (INV) w.y = -w.y;
-                v[q] = cmul(v[q], w);
-            }
+            for (int q = 2; q < R; ++q) w[q] = q % 2 == 0 ? cmul(w[q / 2], w[q / 2]) : cmul(w[q - 1], w[1]);
+#pragma unroll
+            for (int q = 1; q < R; ++q) v[q] = cmul(v[q], w[q]);
         }
         dft<R, INV>(v);
 #pragma unroll
@@ -441,11 +446,12 @@ __global__ void __launch_bounds__(kFftThreads) k_spec_y(SpectralArgs a) {
 // x_k = y_k - au_k P_k x_k+1.  As k_thomas_split: block (32, LPC), warp w holds
 // the run of CH levels from w CH on of 32 neighbouring pairs, so every load is
 // issued at once and a full line wide; the runs' affine maps are chained
-// through shared memory.  A pair shares its pivots (except pair 0).
+// through shared memory by one warp.  A pair shares its pivots (except pair 0).
 template <int CH>
 __global__ void __launch_bounds__(1024) k_spec_z(SpectralArgs a) {
     if (krylov_done(a.scal)) return;
     __shared__ float4 sc[32][32];  // composite of a run: (A.x, A.y, B.x, B.y)
+    __shared__ float2 sin[32][32];  // value entering a run
     const int lane = threadIdx.x, part = threadIdx.y, LPC = blockDim.y;
     const int i = blockIdx.x * 32 + lane, y = blockIdx.y;
     const bool valid = i < a.npair;
@@ -478,12 +484,18 @@ __global__ void __launch_bounds__(1024) k_spec_z(SpectralArgs a) {
     }
     sc[part][lane] = make_float4(A.x, A.y, B.x, B.y);
     __syncthreads();
+    // one warp chains the runs: every warp for itself reads half of all composites
     float2 c = make_float2(0.f, 0.f);
-    for (int w = 0; w < part; ++w) {
-        const float4 f = sc[w][lane];
-        c = make_float2(f.x + f.z * c.x, f.y + f.w * c.y);
+    if (part == 0) {
+#pragma unroll 8
+        for (int w = 0; w < LPC; ++w) {
+            const float4 f = sc[w][lane];
+            sin[w][lane] = c;
+            c = make_float2(f.x + f.z * c.x, f.y + f.w * c.y);
+        }
     }
     __syncthreads();
+    c = sin[part][lane];
 #pragma unroll
     for (int q = 0; q < CH; ++q) {
         const int k = kb + q;
@@ -508,11 +520,17 @@ __global__ void __launch_bounds__(1024) k_spec_z(SpectralArgs a) {
     }
     sc[part][lane] = make_float4(A.x, A.y, B.x, B.y);
     __syncthreads();
-    c = make_float2(0.f, 0.f);
-    for (int w = LPC - 1; w > part; --w) {
-        const float4 f = sc[w][lane];
-        c = make_float2(f.x + f.z * c.x, f.y + f.w * c.y);
+    if (part == 0) {
+        c = make_float2(0.f, 0.f);
+#pragma unroll 8
+        for (int w = LPC - 1; w >= 0; --w) {
+            const float4 f = sc[w][lane];
+            sin[w][lane] = c;
+            c = make_float2(f.x + f.z * c.x, f.y + f.w * c.y);
+        }
     }
+    __syncthreads();
+    c = sin[part][lane];
 #pragma unroll
     for (int q = CH - 1; q >= 0; --q) {
         const int k = kb + q;
