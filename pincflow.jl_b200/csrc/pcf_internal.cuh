@@ -38,6 +38,16 @@ struct NvtxScope {
 
 int pcf_set_cuda_error(cudaError_t e);
 
+// Copies a host array that may go out of scope to the device, ordered before
+// later work on `stream`.  The library's streams do not wait for the default
+// stream (cudaStreamNonBlocking), and cudaMemcpy from pageable memory may
+// return before its device copy is complete, so a plain cudaMemcpy is not
+// ordered before their kernels.
+static inline cudaError_t pcf_upload(void *dst, const void *src, size_t bytes, cudaStream_t stream) {
+    const cudaError_t e = cudaMemcpyAsync(dst, src, bytes, cudaMemcpyHostToDevice, stream);
+    return e != cudaSuccess ? e : cudaStreamSynchronize(stream);
+}
+
 // ------------------------------------------------------- bounds checking --
 // Built with -DPCF_BOUNDS_CHECK (build.py --checked: the library
 // libpincflow_poisson_checked.so), every instrumented global access first

@@ -1223,8 +1223,8 @@ int pcf_gemm_bf16(const unsigned short *A, long long a_len, long long a_rs, long
         rc = pcf_set_cuda_error(e);
     }
     if (!rc) {
-        cudaMemcpy(dA, A, a_len * 2, cudaMemcpyHostToDevice);
-        cudaMemcpy(dB, B, b_len * 2, cudaMemcpyHostToDevice);
+        pcf_upload(dA, A, a_len * 2, 0);
+        pcf_upload(dB, B, b_len * 2, 0);
         cudaMemset(dD, 0, sizeof(float) * (size_t)M * N * ks);
         cudaMemset(derr, 0, sizeof(int));
         pcf::umma::GemmArgs g{};
@@ -1431,7 +1431,7 @@ int pcf_net_forward(pcf_net *w, const double *in, int nx, int ny, int nz, double
     double *d = nullptr;
     PCF_CUDA_TRY(cudaMalloc(&d, 2 * bytes));
     int rc = PCF_OK;
-    if (cudaMemcpy(d, in, bytes, cudaMemcpyHostToDevice) != cudaSuccess) rc = PCF_ECUDA;
+    if (pcf_upload(d, in, bytes, w->n.stream) != cudaSuccess) rc = PCF_ECUDA;
     if (!rc) rc = pcf_net_apply_device(w, d, nx, ny, nz, 1.0, 1.0, 0.0, d + (size_t)nx * ny * nz, 1, nullptr);
     if (!rc && cudaStreamSynchronize(w->n.stream) != cudaSuccess) rc = PCF_ECUDA;
     if (!rc) rc = check_err(w->n);
@@ -1516,8 +1516,8 @@ int pcf_net_gradients(pcf_net *w, const double *b, const double *x, int nx, int 
     float *d = nullptr;
     PCF_CUDA_TRY(cudaMalloc(&d, 2 * cnt * sizeof(float)));
     int rc = PCF_OK;
-    if (cudaMemcpy(d, hb.data(), cnt * 4, cudaMemcpyHostToDevice) != cudaSuccess ||
-        cudaMemcpy(d + cnt, hx.data(), cnt * 4, cudaMemcpyHostToDevice) != cudaSuccess)
+    if (pcf_upload(d, hb.data(), cnt * 4, w->n.stream) != cudaSuccess ||
+        pcf_upload(d + cnt, hx.data(), cnt * 4, w->n.stream) != cudaSuccess)
         rc = PCF_ECUDA;
     if (!rc) rc = pcf_net_train_step(w, d, d + cnt, nx, ny, nz, 0.0, loss, grad);
     cudaFree(d);

@@ -172,7 +172,7 @@ constexpr int stencil_bulk_smem() {
 // planes directly) when the driver has no tensor-map encoder or the grid
 // breaks the copy's alignment rules (x rows of a multiple of 16 bytes, at
 // least one 128-wide box wide).
-static bool make_coef16_maps(const __nv_bfloat16 *coef16, const Dims &d, void *maps) {
+static bool make_coef16_maps(const __nv_bfloat16 *coef16, const Dims &d, void *maps, cudaStream_t stream) {
     using Encode = decltype(&cuTensorMapEncodeTiled);
     static Encode encode = [] {
         void *fn = nullptr;
@@ -198,7 +198,7 @@ static bool make_coef16_maps(const __nv_bfloat16 *coef16, const Dims &d, void *m
                    CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) != CUDA_SUCCESS)
             return false;
     }
-    return cudaMemcpy(maps, host, sizeof(host), cudaMemcpyHostToDevice) == cudaSuccess;
+    return pcf_upload(maps, host, sizeof(host), stream) == cudaSuccess;
 }
 
 // The tensor maps of an FP8 operator copy (25 planes of nx x ny x nz bytes)
@@ -207,7 +207,7 @@ static bool make_coef16_maps(const __nv_bfloat16 *coef16, const Dims &d, void *m
 // 18 planes ALD..AFUU, then [2..3] the same with 64-wide boxes.  False when
 // the grid breaks the alignment rules (rows of a multiple of 16 bytes, at
 // least one 128-wide box wide) or no encoder is available.
-static bool make_coef8_maps(const uint8_t *coef8, const Dims &d, void *maps) {
+static bool make_coef8_maps(const uint8_t *coef8, const Dims &d, void *maps, cudaStream_t stream) {
     using Encode = decltype(&cuTensorMapEncodeTiled);
     static Encode encode = [] {
         void *fn = nullptr;
@@ -233,7 +233,7 @@ static bool make_coef8_maps(const uint8_t *coef8, const Dims &d, void *maps) {
                    CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) != CUDA_SUCCESS)
             return false;
     }
-    return cudaMemcpy(maps, host, sizeof(host), cudaMemcpyHostToDevice) == cudaSuccess;
+    return pcf_upload(maps, host, sizeof(host), stream) == cudaSuccess;
 }
 
 // Raises the staged stencil's dynamic shared-memory limit on the current
@@ -1100,7 +1100,7 @@ static int mg_prepare(pcf_handle *h, const pcf_params *prm, bool ensemble = fals
                 float *c16 = nullptr, *maps = nullptr;
                 if ((rc = alloc(&c16, (C.d.n * PCF_NCOEF + 1) / 2)) || (rc = alloc(&maps, 6 * 128 / 4))) return rc;
                 C.coef16 = reinterpret_cast<__nv_bfloat16 *>(c16);
-                if (make_coef16_maps(C.coef16, C.d, maps)) C.tmap16 = maps;
+                if (make_coef16_maps(C.coef16, C.d, maps, h->stream)) C.tmap16 = maps;
             }
         }
         m.min_columns = prm->mg_min_columns;
@@ -1161,7 +1161,7 @@ static int mg_prepare(pcf_handle *h, const pcf_params *prm, bool ensemble = fals
         const cudaError_t e = cudaMalloc(&maps, 6 * 128);
         if (e != cudaSuccess) return pcf_set_cuda_error(e);
         m.allocs.push_back(maps);
-        if (make_coef16_maps(h->coef16, h->d, maps)) m.lv[0].tmap16 = maps;
+        if (make_coef16_maps(h->coef16, h->d, maps, h->stream)) m.lv[0].tmap16 = maps;
     }
     // the finest level's pseudo-time steps on an FP8 copy of its planes
     // (mg_smoother_fp8), made from the BF16 copy once per operator
@@ -1186,7 +1186,7 @@ static int mg_prepare(pcf_handle *h, const pcf_params *prm, bool ensemble = fals
         const cudaError_t e = cudaMalloc(&maps, 4 * 128);
         if (e != cudaSuccess) return pcf_set_cuda_error(e);
         m.allocs.push_back(maps);
-        if (make_coef8_maps(h->coef8, h->d, maps)) m.maps8 = maps;
+        if (make_coef8_maps(h->coef8, h->d, maps, h->stream)) m.maps8 = maps;
     }
     m.lv[0].tmap8 = fp8 ? m.maps8 : nullptr;
     if (m.lv[0].tmap8 && h->coef8_version != h->op_version) {
@@ -1357,7 +1357,7 @@ static int spectral_create(pcf_handle *h) {
     }
     a.fx.tw = tw;
     a.fy.tw = tw + nx;
-    cudaError_t e = cudaMemcpy(tw, host.data(), sizeof(float2) * host.size(), cudaMemcpyHostToDevice);
+    cudaError_t e = pcf_upload(tw, host.data(), sizeof(float2) * host.size(), h->stream);
     // x: row pairs per block, y: pairs per block; about 2048 values in flight a
     // block, fewer where that leaves less than two blocks per SM
     const long long pairs = (a.rows + 1) / 2;
@@ -3642,7 +3642,7 @@ static int ensemble_capture_loop(pcf_ensemble *e, const pcf_params *prm, int ci,
         PCF_CUDA_TRY(cudaMalloc(&e->d_batches, sizeof(int)));
         std::vector<KrylovScalars *> ptrs(n);
         for (int q = 0; q < n; ++q) ptrs[q] = e->m[q]->scal32;
-        PCF_CUDA_TRY(cudaMemcpy(e->d_scal, ptrs.data(), sizeof(KrylovScalars *) * n, cudaMemcpyHostToDevice));
+        PCF_CUDA_TRY(pcf_upload(e->d_scal, ptrs.data(), sizeof(KrylovScalars *) * n, e->origin));
     }
     cudaGraph_t g = nullptr;
     PCF_CUDA_TRY(cudaGraphCreate(&g, 0));
