@@ -259,6 +259,7 @@ struct pcf_handle {
     pcf::ProfState *prof;
     pcf::ProfAcc prof_acc[PCF_PROF_NTAGS];
     pcf::GraphCache *gcache;
+    long long graph_epoch;       // times clear_graphs ran: what a graph captured before then holds is stale
     long long graph_launches;    // kernels in the graph being replayed
     pcf_net *net;                // learned warm start (not owned)
     pcf::MgState *mg;            // multigrid hierarchy (allocated on first use)

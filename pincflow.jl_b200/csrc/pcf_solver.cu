@@ -1761,8 +1761,9 @@ struct RunOut {
 };
 
 // A batch of BiCGSTAB iterations captured as a CUDA graph.  The kernels'
-// arguments are the handle's fixed buffers and the loop configuration, so one
-// graph per configuration serves every later solve on the handle.
+// arguments are the handle's fixed buffers, its grid spacings (the flux form's)
+// and the loop configuration, so one graph per configuration serves every later
+// solve on the handle until clear_graphs (new spacings, new level buffers).
 struct GraphKey {
     int tsize, precond, pc_iters, flex, reliable, pi, batch;
     double deta;
@@ -1890,7 +1891,10 @@ static int batch_graph(pcf_handle *h, const Work<T> &w, const LoopCfg &c, const 
     return PCF_OK;
 }
 
+// Drops the handle's captured graphs; an ensemble's graph holds the same
+// arguments and is captured anew when a member's epoch has moved.
 static void clear_graphs(pcf_handle *h) {
+    h->graph_epoch += 1;
     if (!h->gcache) return;
     for (const GraphEntry &e : h->gcache->entries) cudaGraphExecDestroy(e.exec);
     h->gcache->entries.clear();
@@ -2289,6 +2293,7 @@ int pcf_set_grid(pcf_handle *h, double dx, double dy, double dz, const double *j
     PCF_CUDA_TRY(cudaSetDevice(h->dims.device));
     int rp = ensure_planes(h);  // of the operator assembled from the fields replaced here
     if (rp) return rp;
+    if (dx != h->dx || dy != h->dy || dz != h->dz) clear_graphs(h);  // captured flux-form applies hold the spacings
     const size_t b = sizeof(double) * (size_t)h->nh;
     h->dx = dx;
     h->dy = dy;
@@ -3564,6 +3569,7 @@ struct pcf_ensemble {
     bool use_sp = false, use_fx = false, key_sp = false, key_fx = false;
     int key_ci = 0, key_precond = 0, key_pc_iters = 0, key_mg = 0, key_mg_ci = 0, key_mg_min = 0, key_maxit = 0;
     double key_dtau = 0, key_mg_dtau = 0;
+    std::vector<long long> key_epoch;   // the members' graph_epoch at the capture
     KrylovScalars *h_status = nullptr;  // pinned, 2 slots x members
     double *h_norm = nullptr;           // pinned, members; then as many words for k_flux_build's findings
     // the whole solve as one graph launch: a conditional WHILE node around
@@ -3691,6 +3697,12 @@ static int ensemble_capture_loop(pcf_ensemble *e, const pcf_params *prm, int ci,
     return PCF_OK;
 }
 
+static std::vector<long long> ensemble_epochs(const pcf_ensemble *e) {
+    std::vector<long long> v;
+    for (const pcf_handle *h : e->m) v.push_back(h->graph_epoch);
+    return v;
+}
+
 static int ensemble_capture(pcf_ensemble *e, const pcf_params *prm, int ci) {
     if (e->exec) {
         cudaGraphExecDestroy(e->exec);
@@ -3722,6 +3734,7 @@ static int ensemble_capture(pcf_ensemble *e, const pcf_params *prm, int ci) {
     e->key_maxit = prm->poisson_iterations;
     e->key_sp = e->use_sp;
     e->key_fx = e->use_fx;
+    e->key_epoch = ensemble_epochs(e);
     return ensemble_capture_loop(e, prm, ci, (prm->poisson_iterations + ci - 1) / ci);
 }
 
@@ -3849,7 +3862,7 @@ int pcf_ensemble_solve_device(pcf_ensemble *e, const double *const *d_rhs, const
         e->key_pc_iters != prm->preconditioner_iterations || e->key_dtau != prm->dtau || e->key_mg != prm->multigrid ||
         e->key_mg_ci != prm->mg_coarse_iterations || e->key_mg_min != prm->mg_min_columns ||
         e->key_mg_dtau != prm->mg_dtau || e->key_maxit != prm->poisson_iterations || e->key_sp != e->use_sp ||
-        e->key_fx != e->use_fx) {
+        e->key_fx != e->use_fx || e->key_epoch != ensemble_epochs(e)) {
         if ((rc = ensemble_capture(e, prm, ci))) return rc;
     }
     std::vector<double> bnorm(n), tol(n);

@@ -1,0 +1,114 @@
+"""GPU: one handle (and one ensemble) used for different calls in turn.
+
+What a handle keeps between calls -- captured iteration graphs, the multigrid
+hierarchy, the operator in flux form or as planes -- must not reach the next
+call's result.  Every kernel sums in a fixed order, so a call on a used handle
+gives the bits of the same call on a new one; the residual is checked with the
+coefficient planes as well (apply_operator), which no solve of the flux form
+shares with it.
+"""
+import numpy as np
+import pytest
+
+from pincflow_poisson import configs as C
+from pincflow_poisson import fields as F
+
+pytestmark = pytest.mark.gpu
+
+KW = dict(tolerance=1e-10, tolerance_is_relative=True, poisson_iterations=4000, precision="mixed", multigrid=True)
+
+
+def _grids():
+    """Two problems of one shape and model with other spacings, metrics and backgrounds."""
+    a = C.c2(nx=48, ny=40, nz=24)
+    b = C.c5(nx=48, ny=40, nz=24, lx=60e3, ly=90e3, ridges=2)
+    for key in ("dx", "dy", "dz"):
+        assert abs(a["fields"][key] / b["fields"][key] - 1) > 0.1
+    return a, b
+
+
+def _handle(pcf, cfg):
+    s = pcf.PoissonSolver(cfg["dom"], cfg["model"])
+    s.set_grid(cfg["fields"])
+    s.set_background(cfg["fields"])
+    return s
+
+
+def _solve(pcf, s, cfg, **nl):
+    dpip = np.zeros(cfg["dom"].halo_shape)
+    info = s.solve_poisson(cfg["rhs"], cfg["rho"], cfg["betar"], cfg["dt"], cfg["rayleigh_factor"], 1.0,
+                           pcf.PoissonNamelist(**dict(KW, **nl)), dpip)
+    return cfg["dom"].interior(dpip).copy(), info
+
+
+def _residual(s, cfg, x):
+    """Relative residual of the pressure x with the coefficient planes."""
+    r = cfg["rhs"] - s.apply_operator(x * F.fcscal(cfg["dom"], cfg["fields"]) * cfg["dt"])
+    return float(np.sqrt((r ** 2).mean() / (cfg["rhs"] ** 2).mean()))
+
+
+@pytest.mark.parametrize("more", [dict()], ids=["spectral"])
+def test_solve_after_another_grid(pcf, more):
+    a, b = _grids()
+    with _handle(pcf, a) as s, _handle(pcf, b) as new:
+        _, first = _solve(pcf, s, a, **more)
+        assert not first.errflag
+        s.set_grid(b["fields"])
+        s.set_background(b["fields"])
+        got, info = _solve(pcf, s, b, **more)
+        want, winfo = _solve(pcf, new, b, **more)
+        assert not info.errflag and not winfo.errflag
+        assert _residual(s, b, got) <= 1.01e-10, _residual(s, b, got)
+        assert info.niter == winfo.niter, (info.niter, winfo.niter)
+        assert np.array_equal(got, want)
+
+
+def test_operator_of_the_last_solve_survives_another_grid(pcf):
+    """The operator is the last solve's until the next one is made, also where
+    the grid has been replaced since."""
+    a, b = _grids()
+    v = np.random.default_rng(3).standard_normal(a["dom"].interior_shape)
+    with _handle(pcf, a) as s, _handle(pcf, a) as ref:
+        _solve(pcf, s, a)
+        s.set_grid(b["fields"])
+        s.set_background(b["fields"])
+        ref.compute_operator(a["rho"], a["betar"], a["dt"], a["rayleigh_factor"], return_coef=False)
+        assert np.array_equal(s.apply_operator(v), ref.apply_operator(v))
+
+
+def _device(cfgs):
+    import torch
+    out = []
+    for cfg in cfgs:
+        d = {k: torch.from_numpy(np.ascontiguousarray(cfg[k])).cuda() for k in ("rhs", "rho", "betar")}
+        d["dpip"] = torch.zeros(cfg["dom"].halo_shape, dtype=torch.float64, device="cuda")
+        out.append(d)
+    return out
+
+
+def _solve_ensemble(pcf, ens, cfgs, **nl):
+    dev = _device(cfgs)
+    infos = ens.solve_poisson_device([d["rhs"].data_ptr() for d in dev], [d["rho"].data_ptr() for d in dev],
+                                     [d["betar"].data_ptr() for d in dev], [c["dt"] for c in cfgs],
+                                     [c["rayleigh_factor"] for c in cfgs], [c["tolref"] for c in cfgs],
+                                     pcf.PoissonNamelist(**dict(KW, **nl)), [d["dpip"].data_ptr() for d in dev])
+    return [c["dom"].interior(d["dpip"].cpu().numpy()).copy() for c, d in zip(cfgs, dev)], infos
+
+
+@pytest.mark.parametrize("more", [dict()], ids=["spectral"])
+def test_ensemble_after_another_grid(pcf, more):
+    a, b = _grids()
+    other = C.c2(nx=32, ny=24, nz=16, seed=9)
+    with _handle(pcf, other) as s0, _handle(pcf, a) as s1, _handle(pcf, other) as n0, _handle(pcf, b) as n1:
+        with pcf.Ensemble([s0, s1]) as used, pcf.Ensemble([n0, n1]) as new:
+            _, infos = _solve_ensemble(pcf, used, [other, a], **more)
+            assert not any(i.errflag for i in infos)
+            s1.set_grid(b["fields"])
+            s1.set_background(b["fields"])
+            got, infos = _solve_ensemble(pcf, used, [other, b], **more)
+            want, winfos = _solve_ensemble(pcf, new, [other, b], **more)
+        assert not any(i.errflag for i in infos)
+        assert _residual(s1, b, got[1]) <= 1.01e-10, _residual(s1, b, got[1])
+        assert [i.niter for i in infos] == [i.niter for i in winfos]
+        for g, w in zip(got, want):
+            assert np.array_equal(g, w)
