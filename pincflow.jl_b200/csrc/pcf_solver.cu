@@ -3567,8 +3567,8 @@ struct pcf_ensemble {
     bool key_valid = false;
     // spectral preconditioner and flux-form operator: this solve's, the captured graph's
     bool use_sp = false, use_fx = false, key_sp = false, key_fx = false;
-    int key_ci = 0, key_precond = 0, key_pc_iters = 0, key_mg = 0, key_mg_ci = 0, key_mg_min = 0, key_maxit = 0;
-    double key_dtau = 0, key_mg_dtau = 0;
+    int key_ci = 0;
+    pcf_params key_prm{};               // the settings the captured graph was recorded with
     std::vector<long long> key_epoch;   // the members' graph_epoch at the capture
     KrylovScalars *h_status = nullptr;  // pinned, 2 slots x members
     double *h_norm = nullptr;           // pinned, members; then as many words for k_flux_build's findings
@@ -3697,6 +3697,16 @@ static int ensemble_capture_loop(pcf_ensemble *e, const pcf_params *prm, int ci,
     return PCF_OK;
 }
 
+// Whether two settings record the same iteration (the other fields are read by
+// the set-up or go into each run's scalar block).
+static bool same_iteration(const pcf_params &a, const pcf_params &b) {
+    return a.preconditioner == b.preconditioner && a.preconditioner_iterations == b.preconditioner_iterations &&
+           a.dtau == b.dtau && a.multigrid == b.multigrid && a.mg_dtau == b.mg_dtau &&
+           a.mg_coarse_iterations == b.mg_coarse_iterations && a.mg_min_columns == b.mg_min_columns &&
+           a.mg_operator_bf16 == b.mg_operator_bf16 && a.mg_fused_coarse == b.mg_fused_coarse &&
+           a.mg_smoother_fp8 == b.mg_smoother_fp8 && a.poisson_iterations == b.poisson_iterations;
+}
+
 static std::vector<long long> ensemble_epochs(const pcf_ensemble *e) {
     std::vector<long long> v;
     for (const pcf_handle *h : e->m) v.push_back(h->graph_epoch);
@@ -3724,14 +3734,7 @@ static int ensemble_capture(pcf_ensemble *e, const pcf_params *prm, int ci) {
     e->graph_launches = nl;
     e->key_valid = true;
     e->key_ci = ci;
-    e->key_precond = prm->preconditioner;
-    e->key_pc_iters = prm->preconditioner_iterations;
-    e->key_dtau = prm->dtau;
-    e->key_mg = prm->multigrid;
-    e->key_mg_ci = prm->mg_coarse_iterations;
-    e->key_mg_min = prm->mg_min_columns;
-    e->key_mg_dtau = prm->mg_dtau;
-    e->key_maxit = prm->poisson_iterations;
+    e->key_prm = *prm;
     e->key_sp = e->use_sp;
     e->key_fx = e->use_fx;
     e->key_epoch = ensemble_epochs(e);
@@ -3858,11 +3861,8 @@ int pcf_ensemble_solve_device(pcf_ensemble *e, const double *const *d_rhs, const
         for (int q = 0; q < n; ++q) PCF_CUDA_TRY(cudaStreamSynchronize(e->m[q]->stream));
     }
     // the iteration graph, captured with every stream idle
-    if (!e->exec || !e->key_valid || e->key_ci != ci || e->key_precond != prm->preconditioner ||
-        e->key_pc_iters != prm->preconditioner_iterations || e->key_dtau != prm->dtau || e->key_mg != prm->multigrid ||
-        e->key_mg_ci != prm->mg_coarse_iterations || e->key_mg_min != prm->mg_min_columns ||
-        e->key_mg_dtau != prm->mg_dtau || e->key_maxit != prm->poisson_iterations || e->key_sp != e->use_sp ||
-        e->key_fx != e->use_fx || e->key_epoch != ensemble_epochs(e)) {
+    if (!e->exec || !e->key_valid || e->key_ci != ci || !same_iteration(e->key_prm, *prm) ||
+        e->key_sp != e->use_sp || e->key_fx != e->use_fx || e->key_epoch != ensemble_epochs(e)) {
         if ((rc = ensemble_capture(e, prm, ci))) return rc;
     }
     std::vector<double> bnorm(n), tol(n);

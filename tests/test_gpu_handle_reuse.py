@@ -16,6 +16,7 @@ from pincflow_poisson import fields as F
 pytestmark = pytest.mark.gpu
 
 KW = dict(tolerance=1e-10, tolerance_is_relative=True, poisson_iterations=4000, precision="mixed", multigrid=True)
+VCYCLE = dict(mg_dtau=2.0)  # away from its default: asks for the V-cycle
 
 
 def _grids():
@@ -112,3 +113,47 @@ def test_ensemble_after_another_grid(pcf, more):
         assert [i.niter for i in infos] == [i.niter for i in winfos]
         for g, w in zip(got, want):
             assert np.array_equal(g, w)
+
+
+@pytest.mark.parametrize("first,second", [(dict(), dict(mg_fused_coarse=False)), (dict(mg_operator_bf16=False), dict()),
+                                          (dict(mg_smoother_fp8=True), dict()), (dict(mg_min_columns=64), dict())],
+                         ids=["fused", "bf16", "fp8", "levels"])
+def test_ensemble_after_other_vcycle_settings(pcf, first, second):
+    """One ensemble, its V-cycle with one setting after another: each solve
+    runs the V-cycle that it asks for (as on new handles)."""
+    cfgs = [C.c3(1, nx=32, ny=24, nz=16), C.c3(9, nx=160, ny=16, nz=20)]
+    used = [_handle(pcf, c) for c in cfgs]
+    try:
+        with pcf.Ensemble(used) as ens:
+            for more in (first, second, first):
+                got, infos = _solve_ensemble(pcf, ens, cfgs, **VCYCLE, **more)
+                new = [_handle(pcf, c) for c in cfgs]
+                with pcf.Ensemble(new) as fresh:
+                    want, winfos = _solve_ensemble(pcf, fresh, cfgs, **VCYCLE, **more)
+                for s in new:
+                    s.close()
+                assert not any(i.errflag for i in infos)
+                assert [i.niter for i in infos] == [i.niter for i in winfos]
+                for g, w in zip(got, want):
+                    assert np.array_equal(g, w)
+    finally:
+        for s in used:
+            s.close()
+
+
+def test_ensemble_after_a_members_own_solve(pcf):
+    """A member that solves by itself with another hierarchy in between has
+    freed the level buffers that the ensemble's graph was recorded with."""
+    cfgs = [C.c3(1, nx=32, ny=24, nz=16), C.c3(2, nx=48, ny=32, nz=16)]
+    used = [_handle(pcf, c) for c in cfgs]
+    try:
+        with pcf.Ensemble(used) as ens:
+            want, winfos = _solve_ensemble(pcf, ens, cfgs, **VCYCLE)
+            assert not _solve(pcf, used[1], cfgs[1], mg_min_columns=100)[1].errflag
+            got, infos = _solve_ensemble(pcf, ens, cfgs, **VCYCLE)
+        assert not any(i.errflag for i in infos) and [i.niter for i in infos] == [i.niter for i in winfos]
+        for g, w in zip(got, want):
+            assert np.array_equal(g, w)
+    finally:
+        for s in used:
+            s.close()
