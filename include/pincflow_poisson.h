@@ -137,7 +137,9 @@ typedef struct {
                                       take the spectral preconditioner in its place (the inverse of the operator
                                       averaged over each level: 4-10 iterations) while mg_dtau,
                                       mg_coarse_iterations, mg_min_columns, mg_operator_bf16 and mg_smoother_fp8
-                                      are the defaults, no learned stage runs, nx, ny <= 4096 and nz <= 512; a
+                                      are the defaults, no learned stage runs, nx, ny <= 4096, nz <= 512 and the
+                                      columns make at most 16384 tiles of 32 x 4 (2,097,152 columns, fewer where
+                                      nx, ny are no multiples of these) and the cells number fewer than 2^29; a
                                       solve that has not converged after 24 such iterations goes on with the
                                       V-cycle.  pcf_bicgstab always runs the V-cycle.  inner_tolerance counts
                                       squared there: an update every second iteration instead of each */

@@ -1266,6 +1266,12 @@ struct SpectralState {
     std::vector<void *> allocs;
 };
 
+// Tiles of columns of the flux-form apply: a block each at the least, so their
+// number is bounded by the partial sums of its reductions.
+static long long flux_tiles(const Dims &d) {
+    return ((d.nx + kFluxTX - 1) / kFluxTX) * (long long)((d.ny + kFluxTY - 1) / kFluxTY);
+}
+
 // Whether a solve may replace the V-cycle by the spectral preconditioner: the
 // V-cycle's own settings are the defaults (others ask for that V-cycle), no
 // network takes part (trained on the V-cycle and the planes), and extents the
@@ -1279,7 +1285,8 @@ static bool spectral_applies(const pcf_handle *h, const pcf_params *prm) {
            prm->mg_smoother_fp8 == def.mg_smoother_fp8 && !(prm->learned && h->net) && !h->test_stall &&
            (!prm->preconditioner || prm->preconditioner_iterations >= 1) &&
            h->d.nx <= kFftMaxLength && h->d.ny <= kFftMaxLength && h->d.nz <= kSpectralMaxLevels &&
-           h->d.n < (1LL << 29);  // the flux-form apply's 32-bit byte offsets
+           h->d.n < (1LL << 29) &&  // the flux-form apply's 32-bit byte offsets
+           flux_tiles(h->d) <= kMaxPartials;
 }
 
 static void spectral_free(pcf_handle *h) {
@@ -1436,8 +1443,7 @@ static int flux_apply(pcf_handle *h, FluxArgs<T> a) {
     a.rdy = 1.0 / h->dy;
     a.rdz = 1.0 / h->dz;
     a.diag = h->dims.model == PCF_MODEL_COMPRESSIBLE;
-    const long long gx = (a.nx + kFluxTX - 1) / kFluxTX, gy = (a.ny + kFluxTY - 1) / kFluxTY, xy = gx * gy;
-    if (gy > 65535) return PCF_ERANGE;
+    const long long gx = (a.nx + kFluxTX - 1) / kFluxTX, gy = (a.ny + kFluxTY - 1) / kFluxTY, xy = flux_tiles(h->d);
     // levels per block: about 24 blocks per SM, so that the last of the 5
     // resident waves matters little, and at least 4 levels, as each chunk
     // evaluates one more; 2 on grids that leave the GPU mostly idle
@@ -1446,7 +1452,7 @@ static int flux_apply(pcf_handle *h, FluxArgs<T> a) {
     kc = std::min<long long>(kc, a.nz);
     while (kc < a.nz && xy * ((a.nz + kc - 1) / kc) > kMaxPartials) kc = std::min<long long>(2 * kc, a.nz);
     const long long gz = (a.nz + kc - 1) / kc;
-    if (xy * gz > kMaxPartials) return PCF_ERANGE;
+    if (xy * gz > kMaxPartials) return PCF_ERANGE;  // spectral_applies lets no such grid in
     ProfScope ps(h, a.guard_update ? PCF_PROF_RELIABLE : sizeof(T) == 4 ? PCF_PROF_APPLY32 : PCF_PROF_APPLY64,
                  a.guard_update ? 0.0 : flux_words(h) * sizeof(T) * (double)a.n);
     k_flux_apply<T, EPI><<<dim3((unsigned)gx, (unsigned)gy, (unsigned)gz), dim3(kFluxTX, kFluxTY), 0, h->stream>>>(
