@@ -263,6 +263,9 @@ struct pcf_handle {
     long long graph_launches;    // kernels in the graph being replayed
     pcf_net *net;                // learned warm start (not owned)
     pcf::MgState *mg;            // multigrid hierarchy (allocated on first use)
+    // 1: a multigrid solve ran without building its hierarchy (the spectral
+    // preconditioner took the V-cycle's place); pcf_multigrid_operator builds it
+    int mg_owed;
     pcf::SpectralState *spec;    // spectral preconditioner (allocated on first use)
     float *lr32;                 // learned preconditioner stage: residual and correction (2 n, on first use)
     long long op_version;        // incremented whenever the operator changes

@@ -1205,6 +1205,7 @@ static int mg_prepare(pcf_handle *h, const pcf_params *prm, bool ensemble = fals
     // the finest level's pivots are the handle's (shared with the reference preconditioner)
     int rc = ensure_factors(h, m.lv[0].deta);
     if (rc) return rc;
+    h->mg_owed = 0;
     if (m.version == h->op_version && m.dtau == prm->mg_dtau) return PCF_OK;
     // finest level: fcscal in FP32
     {
@@ -2398,6 +2399,7 @@ static int assemble_chunks(pcf_handle *h, double dt, double rf, int damp_h, int 
             h->op_version += 1;
             h->fac_deta = std::nan("");
             h->flux_only = 1;
+            h->mg_owed = 1;
             h->flux_dt = dt;
             h->flux_rf = rf;
             h->flux_damp = damp_h;
@@ -2584,10 +2586,16 @@ int pcf_multigrid_levels(pcf_handle *h, const pcf_params *prm, int cap, int *nle
 }
 
 int pcf_multigrid_operator(pcf_handle *h, int level, double *coef) {
-    if (!h || !coef || !h->mg || level < 0 || level >= (int)h->mg->lv.size()) return PCF_EINVAL;
+    if (!h || !coef || level < 0) return PCF_EINVAL;
     PCF_CUDA_TRY(cudaSetDevice(h->dims.device));
-    const int rc = ensure_planes(h);
+    int rc = ensure_planes(h);
     if (rc) return rc;
+    if (h->mg_owed) {  // spectral solves run with the default settings only
+        pcf_params def;
+        pcf_params_default(&def);
+        if ((rc = mg_prepare(h, &def))) return rc;
+    }
+    if (!h->mg || level >= (int)h->mg->lv.size()) return PCF_EINVAL;
     const MgLevel &L = h->mg->lv[level];
     const long long m = L.d.n * PCF_NCOEF;
     if (level == 0) {

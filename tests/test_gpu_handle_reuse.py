@@ -35,6 +35,17 @@ def _handle(pcf, cfg):
     return s
 
 
+def _with_density(pcf, cfg, amplitude):
+    """cfg with a density fluctuation and a right-hand side in the range of its operator."""
+    k = np.arange(cfg["dom"].halo_shape[0])[:, None, None]
+    c = dict(cfg, rho=np.ascontiguousarray(amplitude * cfg["fields"]["rhobar"] * np.cos(k)))
+    x = np.random.default_rng(7).standard_normal(cfg["dom"].interior_shape)
+    with _handle(pcf, c) as s:
+        s.compute_operator(c["rho"], c["betar"], c["dt"], c["rayleigh_factor"], return_coef=False)
+        c["rhs"] = s.apply_operator(x)
+    return c
+
+
 def _solve(pcf, s, cfg, **nl):
     dpip = np.zeros(cfg["dom"].halo_shape)
     info = s.solve_poisson(cfg["rhs"], cfg["rho"], cfg["betar"], cfg["dt"], cfg["rayleigh_factor"], 1.0,
@@ -157,3 +168,18 @@ def test_ensemble_after_a_members_own_solve(pcf):
     finally:
         for s in used:
             s.close()
+
+
+def test_multigrid_operator_after_a_solve(pcf):
+    """pcf_multigrid_operator after a multigrid solve: the hierarchy of that
+    solve's operator, whichever preconditioner the solve ran."""
+    cfg = C.c2(nx=48, ny=40, nz=24)
+    nl = pcf.PoissonNamelist(**KW)
+    with _handle(pcf, cfg) as s, _handle(pcf, cfg) as ref:
+        for c in (cfg, _with_density(pcf, cfg, 0.1)):  # a second operator on the same handle
+            assert not _solve(pcf, s, c)[1].errflag
+            ref.compute_operator(c["rho"], c["betar"], c["dt"], c["rayleigh_factor"], return_coef=False)
+            levels = ref.multigrid_levels(nl)
+            for lv in (1, len(levels) - 1, 0):
+                got, want = s.multigrid_operator(lv, levels[lv]), ref.multigrid_operator(lv, levels[lv])
+                assert np.array_equal(got, want), lv
