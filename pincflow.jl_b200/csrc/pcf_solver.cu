@@ -1992,7 +1992,7 @@ static int bicgstab_run(pcf_handle *h, const Work<T> &w, const T *b, double tol,
                         int restart_every = 0, double start = 0.0) {
     int rc0 = run_start<T>(h, w, b, tol, maxit, c, hist_off, hist_scale, bnorm64, ru_delta, restart_every, start);
     if (rc0) return rc0;
-    if (c.sp && !h->prof_on) {
+    if (c.sp && !h->prof_on && maxit > 0) {  // (a WHILE node runs its body at least once)
         cudaGraphExec_t loop = nullptr;
         const int rc = batch_graph<T>(h, w, c, graph_key(h, (int)sizeof(T), c, w.post != nullptr, 0), &loop);
         if (rc) return rc;

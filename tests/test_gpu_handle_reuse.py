@@ -183,3 +183,11 @@ def test_multigrid_operator_after_a_solve(pcf):
             for lv in (1, len(levels) - 1, 0):
                 got, want = s.multigrid_operator(lv, levels[lv]), ref.multigrid_operator(lv, levels[lv])
                 assert np.array_equal(got, want), lv
+
+
+def test_no_iterations_allowed(pcf):
+    cfg = C.c2(nx=48, ny=40, nz=24)
+    with _handle(pcf, cfg) as s:
+        for more in (dict(), VCYCLE):
+            x, info = _solve(pcf, s, cfg, poisson_iterations=0, **more)
+            assert info.errflag and info.niter == 0 and not x.any(), (more, info)
