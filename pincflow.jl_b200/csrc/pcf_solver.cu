@@ -1061,8 +1061,6 @@ static int mg_prepare(pcf_handle *h, const pcf_params *prm, bool ensemble = fals
         mg_free(h);
         MgLevel L0;
         L0.d = h->d;
-        L0.dx = h->dx;
-        L0.dy = h->dy;
         m.lv.push_back(L0);
         for (;;) {
             const MgLevel &F = m.lv.back();
@@ -1077,8 +1075,6 @@ static int mg_prepare(pcf_handle *h, const pcf_params *prm, bool ensemble = fals
             C.d.n = (long long)C.d.plane * C.d.nz;
             C.cx = cx;
             C.cy = cy;
-            C.dx = F.dx * cx;
-            C.dy = F.dy * cy;
             m.lv.push_back(C);
         }
         auto alloc = [&](float **p, long long count) -> int {
@@ -1200,6 +1196,12 @@ static int mg_prepare(pcf_handle *h, const pcf_params *prm, bool ensemble = fals
         h->launches += 3;
         PCF_CUDA_TRY(cudaGetLastError());
         h->coef8_version = h->op_version;
+    }
+    // the spacings are the current grid's (pcf_set_grid may have changed them since the levels were laid out)
+    for (size_t l = 0; l < m.lv.size(); ++l) {
+        MgLevel &L = m.lv[l];
+        L.dx = l == 0 ? h->dx : m.lv[l - 1].dx * L.cx;
+        L.dy = l == 0 ? h->dy : m.lv[l - 1].dy * L.cy;
     }
     for (MgLevel &L : m.lv) L.deta = prm->mg_dtau / (2 * (1 / (L.dx * L.dx) + 1 / (L.dy * L.dy)));
     // the finest level's pivots are the handle's (shared with the reference preconditioner)
@@ -2300,7 +2302,10 @@ int pcf_set_grid(pcf_handle *h, double dx, double dy, double dz, const double *j
     PCF_CUDA_TRY(cudaSetDevice(h->dims.device));
     int rp = ensure_planes(h);  // of the operator assembled from the fields replaced here
     if (rp) return rp;
-    if (dx != h->dx || dy != h->dy || dz != h->dz) clear_graphs(h);  // captured flux-form applies hold the spacings
+    if (dx != h->dx || dy != h->dy || dz != h->dz) {
+        clear_graphs(h);                 // captured flux-form applies hold the spacings
+        if (h->mg) h->mg->version = -1;  // and the V-cycle's pivots their pseudo-time steps
+    }
     const size_t b = sizeof(double) * (size_t)h->nh;
     h->dx = dx;
     h->dy = dy;

@@ -59,7 +59,7 @@ def _residual(s, cfg, x):
     return float(np.sqrt((r ** 2).mean() / (cfg["rhs"] ** 2).mean()))
 
 
-@pytest.mark.parametrize("more", [dict()], ids=["spectral"])
+@pytest.mark.parametrize("more", [dict(), VCYCLE], ids=["spectral", "vcycle"])
 def test_solve_after_another_grid(pcf, more):
     a, b = _grids()
     with _handle(pcf, a) as s, _handle(pcf, b) as new:
@@ -107,7 +107,7 @@ def _solve_ensemble(pcf, ens, cfgs, **nl):
     return [c["dom"].interior(d["dpip"].cpu().numpy()).copy() for c, d in zip(cfgs, dev)], infos
 
 
-@pytest.mark.parametrize("more", [dict()], ids=["spectral"])
+@pytest.mark.parametrize("more", [dict(), VCYCLE], ids=["spectral", "vcycle"])
 def test_ensemble_after_another_grid(pcf, more):
     a, b = _grids()
     other = C.c2(nx=32, ny=24, nz=16, seed=9)
