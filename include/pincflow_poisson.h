@@ -351,6 +351,14 @@ int pcf_apply_multigrid(pcf_handle *h, const double *sin, double *sout, const pc
  * beyond nx, ny = 4096 or nz = 512 (such solves run the V-cycle). */
 int pcf_apply_spectral(pcf_handle *h, const double *sin, double *sout);
 
+/* The operator in flux form, in which spectral solves assemble and apply it,
+ * applied once: out = A (fcscal pi) for the operator of the last solve, with
+ * the FP64 values or (PCF_PRECISION_FP32) the FP32 copy (host FP64 arrays,
+ * nx*ny*nz).  Halo columns count as the periodic image of the interior.
+ * PCF_ENOTREADY where that operator is held as coefficient planes (another
+ * kind of solve, or a call since that needed them). */
+int pcf_apply_flux(pcf_handle *h, const double *pi, double *out, int precision);
+
 /* Stencil tile autotuner (no reference counterpart).  One entry per device,
  * kernel family and grid size that a solve with pcf_params.autotune = 1 has
  * tuned: the chosen tile (tile_x threads along x, 128 threads per block, vec

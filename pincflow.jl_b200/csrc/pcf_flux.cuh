@@ -225,8 +225,9 @@ __global__ void __launch_bounds__(kFluxTX *kFluxTY, sizeof(T) == 4 ? 4 : 2) k_fl
             pd[d] = pi(d, max(ks - 1, 0));
             pc[d] = pi(d, ks);
             pu[d] = pi(d, ks + 1);
-            // ks < top (nz >= 4); one-sided at the bottom
-            e[d] = ks == 0 ? T(4) * pu[d] - T(3) * pc[d] - pi(d, 2) : pu[d] - pd[d];
+            // ks < top (nz >= 4); one-sided at the bottom, as differences (-3, 4, -1
+            // written out rounds 3 pi, so a constant would not give zero)
+            e[d] = ks == 0 ? T(3) * (pu[d] - pc[d]) - (pi(d, 2) - pu[d]) : pu[d] - pd[d];
         }
         fluxes(N.L, pc, e);
         T m13k = N.L.m13[0], m23k = N.L.m23[0];
@@ -241,8 +242,9 @@ __global__ void __launch_bounds__(kFluxTX *kFluxTY, sizeof(T) == 4 ? 4 : 2) k_fl
             const bool last = k + 2 > top;  // level k + 1 is the top one: one-sided
 #pragma unroll
             for (int d = 0; d < 5; ++d) {
-                q[d] = C.th[d] * (pc[d] - pu[d]) + pu[d];
-                e[d] = last ? T(3) * pu[d] - T(4) * pc[d] + pd[d] : C.up[d] - pc[d];
+                const T up = pu[d] - pc[d];
+                q[d] = pu[d] - C.th[d] * up;
+                e[d] = last ? T(3) * up - (pc[d] - pd[d]) : C.up[d] - pc[d];
                 pd[d] = pc[d];
                 pc[d] = pu[d];
                 pu[d] = C.up[d];

@@ -2649,6 +2649,34 @@ int pcf_apply_spectral(pcf_handle *h, const double *sin_, double *sout) {
     return PCF_OK;
 }
 
+int pcf_apply_flux(pcf_handle *h, const double *pi, double *out, int precision) {
+    if (!h || !pi || !out || (precision != PCF_PRECISION_FP64 && precision != PCF_PRECISION_FP32)) return PCF_EINVAL;
+    if (!h->operator_set || !h->flux_only) return PCF_ENOTREADY;
+    PCF_CUDA_TRY(cudaSetDevice(h->dims.device));
+    const bool f32 = precision == PCF_PRECISION_FP32;
+    int rc = upload_vec(h, pi, h->b64, f32 ? h->s32 : nullptr);
+    if (rc) return rc;
+    if (f32) {
+        FluxArgs<float> a;
+        a.s = a.w1 = h->s32;
+        a.out = h->v32;
+        a.red = red(h, nullptr, FIN_STORE, h->dot_out);
+        if ((rc = flux_apply<float, EPI_DOT1>(h, a))) return rc;
+        k_to_double<<<vec_grid(h->d.n), 256, 0, h->stream>>>(h->v32, h->w64, h->d.n);
+        h->launches += 1;
+        PCF_CUDA_TRY(cudaGetLastError());
+    } else {
+        FluxArgs<double> a;
+        a.s = a.w1 = h->b64;
+        a.out = h->w64;
+        a.red = red(h, nullptr, FIN_STORE, h->dot_out);
+        if ((rc = flux_apply<double, EPI_DOT1>(h, a))) return rc;
+    }
+    PCF_CUDA_TRY(cudaMemcpyAsync(out, h->w64, sizeof(double) * h->d.n, cudaMemcpyDeviceToHost, h->stream));
+    PCF_CUDA_TRY(cudaStreamSynchronize(h->stream));
+    return PCF_OK;
+}
+
 int pcf_autotune_entries(pcf_tune_entry *out, int cap, int *count) {
     if (!count || cap < 0 || (cap > 0 && !out)) return PCF_EINVAL;
     std::lock_guard<std::mutex> lk(g_tune_mu);

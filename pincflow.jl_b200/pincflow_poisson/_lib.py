@@ -39,6 +39,7 @@ EXPORTS = [
     "pcf_set_operator", "pcf_apply_operator", "pcf_apply_preconditioner", "pcf_bicgstab",
     "pcf_global_dot", "pcf_device_bytes", "pcf_launch_count", "pcf_profile_enable", "pcf_profile_read",
     "pcf_residual_history", "pcf_multigrid_levels", "pcf_multigrid_operator", "pcf_apply_multigrid", "pcf_apply_spectral",
+    "pcf_apply_flux",
     "pcf_autotune_entries", "pcf_autotune_clear", "pcf_ensemble_create", "pcf_ensemble_destroy",
     "pcf_ensemble_solve_device", "pcf_ensemble_launch_count", "pcf_compute_lhs", "pcf_compute_lhs_device",
     "pcf_correct", "pcf_correct_device", "pcf_apply_corrector_device",
@@ -140,6 +141,7 @@ def load(path: str | None = None):
     lib.pcf_multigrid_operator.argtypes = [vp, ctypes.c_int, dp]
     lib.pcf_apply_multigrid.argtypes = [vp, dp, dp, P(PcfParams)]
     lib.pcf_apply_spectral.argtypes = [vp, dp, dp]
+    lib.pcf_apply_flux.argtypes = [vp, dp, dp, ctypes.c_int]
     lib.pcf_autotune_entries.argtypes = [P(PcfTuneEntry), ctypes.c_int, P(ctypes.c_int)]
     lib.pcf_autotune_clear.argtypes = []
     lib.pcf_compute_lhs.argtypes = [vp, dp, dp, dp, dp, dp, dp]

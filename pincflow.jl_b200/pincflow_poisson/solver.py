@@ -386,6 +386,14 @@ class PoissonSolver:
         _lib.check(self.lib.pcf_apply_spectral(self._h, _lib.dptr(_f64(sin)), _lib.dptr(out)), "pcf_apply_spectral")
         return out
 
+    def apply_flux(self, pi, precision="fp64"):
+        """A (fcscal pi) with the operator in flux form that the last spectral
+        solve assembled (an error where the handle holds it as planes)."""
+        out = np.zeros(self.dom.interior_shape)
+        _lib.check(self.lib.pcf_apply_flux(self._h, _lib.dptr(_f64(pi)), _lib.dptr(out), _lib.PRECISION[precision]),
+                   "pcf_apply_flux")
+        return out
+
     def apply_bicgstab(self, rhs, tolref, namelist: PoissonNamelist):
         sol = np.zeros(self.dom.interior_shape)
         res = _lib.PcfResult()

@@ -140,3 +140,57 @@ def test_spectral_solve_falls_back_to_the_vcycle(pcf):
             counts.append(info.niter)
     print("iterations with the fallback / V-cycle alone:", counts)
     assert counts[0] > 24, counts
+
+
+def _after_a_solve(pcf, cfg):
+    """A handle whose operator is held in flux form (a default multigrid solve, one iteration)."""
+    s = pcf.PoissonSolver(cfg["dom"], cfg["model"])
+    s.set_grid(cfg["fields"])
+    s.set_background(cfg["fields"])
+    s.solve_poisson(np.ascontiguousarray(cfg["rhs"]), cfg["rho"], cfg["betar"], cfg["dt"], cfg["rayleigh_factor"], 1.0,
+                    pcf.PoissonNamelist(precision="mixed", multigrid=True, poisson_iterations=1,
+                                        damp_horizontal_wind_on_rhs=cfg.get("damp", False)),
+                    np.zeros(cfg["dom"].halo_shape), p=cfg.get("p"))
+    return s
+
+
+def _periodic(dom, a):
+    """a with the periodic image of the interior in its halo columns."""
+    i = (np.arange(dom.nx + 6) - 3) % dom.nx + 3
+    j = (np.arange(dom.ny + 6) - 3) % dom.ny + 3
+    return np.ascontiguousarray(a[:, j][:, :, i])
+
+
+@pytest.mark.parametrize("name", ["mtn", "odd", "rho", "comp", "wide", "wide2"])
+def test_flux_form_matches_the_planes(name, pcf):
+    """The flux form against the coefficient planes, both from the same fields
+    (with even halos).  A coefficient is a product of about 20 factors and a
+    sum of a few such products, which cancel in the row's sum: 1e-13 of the
+    largest result in FP64, 2^29 times as much, 5e-5, in FP32."""
+    cfg = dict(case(name))
+    dom = cfg["dom"]
+    for key in ("rho", "betar", "p"):
+        if cfg[key] is not None:
+            cfg[key] = _periodic(dom, cfg[key])
+    pi = np.random.default_rng(5).standard_normal(dom.interior_shape)
+    with _after_a_solve(pcf, cfg) as s:
+        got = s.apply_flux(pi)
+        got32 = s.apply_flux(pi, "fp32")
+        want = s.apply_operator(pi * F.fcscal(dom, cfg["fields"]))
+        with pytest.raises(pcf.PoissonError) as e:  # apply_operator assembled the planes
+            s.apply_flux(pi)
+        assert e.value.code == pcf._lib.PCF_ENOTREADY
+    print(f"{name}: {rel_err(got, want):.1e} {rel_err(got32, want):.1e}")
+    assert rel_err(got, want) <= 1e-13 and rel_err(got32, want) <= 5e-5
+
+
+@pytest.mark.parametrize("name", ["mtn", "odd", "wide", "wide2"])
+def test_flux_form_of_a_constant_is_zero(name, pcf):
+    """Exactly, in either precision and also where multiples of the constant
+    round: every term is a difference of pressures."""
+    cfg = case(name)
+    with _after_a_solve(pcf, cfg) as s:
+        for value in (1.0, 1 / 3, -0.7e5, np.pi):
+            pi = np.full(cfg["dom"].interior_shape, value)
+            for precision in ("fp64", "fp32"):
+                assert not s.apply_flux(pi, precision).any(), (value, precision)
