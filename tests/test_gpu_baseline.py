@@ -9,9 +9,11 @@ which committed a fingerprint of its converged pressure dpip: the values at
 65,536 seeded interior cells, the mean, and the RMS of every z-level with the
 mean removed.  Each test here solves the same workload through the host-array
 entry point pcf_solve (PoissonSolver.solve_poisson) with the default method
-(FP32 BiCGSTAB with the multigrid preconditioner inside FP64 refinement) and,
-on c2, with the plain FP64 method; the c4 members are solved together by the
-ensemble entry point on device arrays.
+(FP32 BiCGSTAB with the spectral preconditioner and the operator in flux form
+inside FP64 refinement), with the V-cycle in its place (BF16 copies, a
+pseudo-time step that is not the default) and, on c2, with the plain FP64
+method; the c4 members are solved together by the ensemble entry point on
+device arrays, likewise with either preconditioner.
 
 Both solves leave the constant (null-space) component of dpip free, so the
 mean difference over the sampled cells is removed first.  Tolerances:
@@ -62,12 +64,15 @@ def _solve(pcf, cfg, **nl):
     return dom.interior(dpip).copy(), info
 
 
-@pytest.mark.parametrize("name,method", [("c2", "mg"), ("c2", "fp64"), ("c5", "mg")])
+@pytest.mark.parametrize("name,method", [("c2", "mg"), ("c2", "fp64"), ("c5", "mg"), ("c2", "vcycle"),
+                                         ("c5", "vcycle")])
 def test_pressure_matches_oracle_fingerprint(pcf, name, method):
     fp = _fingerprint(name)
     cfg = C.c2() if name == "c2" else C.c5()
     assert tuple(fp["shape"]) == cfg["dom"].interior_shape
     nl = dict(precision="fp64") if method == "fp64" else dict(precision="mixed", multigrid=True)
+    if method == "vcycle":
+        nl["mg_dtau"] = 2.4
     dpip, info = _solve(pcf, cfg, **nl)
     assert not info.errflag
     assert info.true_residual <= 1e-10
@@ -76,9 +81,11 @@ def test_pressure_matches_oracle_fingerprint(pcf, name, method):
           f"{info.true_residual:.2e}, max pointwise deviation {dev:.2e}, level RMS {lev:.2e}")
     assert dev <= 1e-6
     assert lev <= 1e-6
+    assert method == "fp64" or (info.niter > 8) == (method == "vcycle"), info.niter
 
 
-def test_c4_ensemble_matches_oracle_fingerprints(pcf):
+@pytest.mark.parametrize("more", [dict(), dict(mg_dtau=2.4)], ids=["spectral", "vcycle"])
+def test_c4_ensemble_matches_oracle_fingerprints(pcf, more):
     """The 32-member c4 ensemble solved together (one graph launch for the
     whole iteration): the first member of each size class against the
     oracle's FP64 solve of that member (tests/golden/c4_<nx>_fp64_fingerprint.npz),
@@ -87,7 +94,7 @@ def test_c4_ensemble_matches_oracle_fingerprints(pcf):
     sizes = C.c4_sizes()
     fps = {nx: _fingerprint(f"c4_{nx}") for nx in sorted(set(sizes))}
     nl = pcf.PoissonNamelist(tolerance=1e-10, tolerance_is_relative=True, poisson_iterations=4000,
-                             precision="mixed", multigrid=True, residual="true")
+                             precision="mixed", multigrid=True, residual="true", **more)
     members = []
     try:
         for q, nx in enumerate(sizes):

@@ -191,3 +191,21 @@ def test_no_iterations_allowed(pcf):
         for more in (dict(), VCYCLE):
             x, info = _solve(pcf, s, cfg, poisson_iterations=0, **more)
             assert info.errflag and info.niter == 0 and not x.any(), (more, info)
+
+
+def test_methods_in_turn_on_one_handle(pcf):
+    """Spectral, V-cycle and FP64 solves in turn, each with another density,
+    give what they give on a new handle."""
+    cfg = C.c2(nx=48, ny=40, nz=24)
+    with _handle(pcf, cfg) as s:
+        for q, more in enumerate([dict(), VCYCLE, dict(), dict(precision="fp64", multigrid=False), dict(), VCYCLE]):
+            c = _with_density(pcf, cfg, 0.02 * (q + 1))
+            got, info = _solve(pcf, s, c, **more)
+            with _handle(pcf, cfg) as new:
+                want, winfo = _solve(pcf, new, c, **more)
+            assert not info.errflag and info.niter == winfo.niter, (q, info, winfo)
+            assert np.array_equal(got, want), q
+            if q % 2:  # the component entry point on the operator that the solve left
+                x, binfo = s.apply_bicgstab(c["rhs"], 1.0, pcf.PoissonNamelist(**dict(KW, multigrid=False)))
+                r = c["rhs"] - s.apply_operator(x)
+                assert not binfo.errflag and np.sqrt((r ** 2).mean() / (c["rhs"] ** 2).mean()) <= 1.01e-10

@@ -139,7 +139,8 @@ def test_spectral_solve_falls_back_to_the_vcycle(pcf):
             assert not info.errflag and info.true_residual <= 1e-8, (more, info)
             counts.append(info.niter)
     print("iterations with the fallback / V-cycle alone:", counts)
-    assert counts[0] > 24, counts
+    # BiCGSTAB counts move by a few iterations with the pseudo-time step and the start
+    assert 24 < counts[0] <= 24 + counts[1] + max(8, 0.15 * counts[1]), counts
 
 
 def _after_a_solve(pcf, cfg):
