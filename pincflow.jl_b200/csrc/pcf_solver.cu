@@ -3523,6 +3523,9 @@ long long pcf_launch_count(const pcf_handle *h) { return h ? h->launches : 0; }
 
 int pcf_set_network(pcf_handle *h, pcf_net *net) {
     if (!h) return PCF_EINVAL;
+    // captured iterations hold the previous network's buffers, and a new network
+    // may have the address of a destroyed one (GraphKey::net)
+    clear_graphs(h);
     h->net = net;
     return PCF_OK;
 }

@@ -247,3 +247,30 @@ def test_unhelpful_stage_costs_a_bounded_number_of_iterations(netmod, scale):
         _, on = s.apply_bicgstab(cfg["rhs"], 1.0, pcf.PoissonNamelist(learned=2, **kw))
     assert not on.errflag and on.true_residual <= 1e-10, on
     assert on.niter <= off.niter + 60 + 8, (on.niter, off.niter)
+
+
+def test_another_network_takes_a_destroyed_ones_place(netmod):
+    """A network attached after the first one was destroyed (whose address it
+    may have): the stage runs with its weights, as on a new handle."""
+    learned, NO = netmod
+    import pincflow_poisson as pcf
+    from pincflow_poisson import configs as C
+    cfg = C.c3(102, nx=32, ny=32, nz=64)
+    nl = pcf.PoissonNamelist(tolerance=1e-8, tolerance_is_relative=True, poisson_iterations=400, precision="mixed",
+                             multigrid=True, learned=2)
+
+    def solve(s, seed):
+        with learned.LearnedNet(max_columns=32 * 32) as net:
+            net.set_params(_random_params(NO, seed) * 0.25)
+            net.set_bias_free(True)
+            s.attach_network(net)
+            x, info = s.apply_bicgstab(cfg["rhs"], 1.0, nl)
+            s.attach_network(None)
+        return x, info
+
+    with _solver(pcf, cfg) as s:
+        for seed in (13, 14, 15):
+            got, info = solve(s, seed)
+            with _solver(pcf, cfg) as new:
+                want, winfo = solve(new, seed)
+            assert info.niter == winfo.niter and np.array_equal(got, want), (seed, info, winfo)
