@@ -501,7 +501,7 @@ int pcf_launch_assemble(pcf_handle *h, double dt, double rf, int damp_h, int c0,
     // a block takes about 6 us per level, whatever the grid (64x64x32: 64 blocks
     // of 16 levels, 107 us)
     a.kpb = pcf::AKC;
-    while (a.kpb > 2 && (long long)gx * gy * ((a.l1 - a.l0 + a.kpb - 1) / a.kpb) < 2 * 148) a.kpb /= 2;
+    while (a.kpb > 2 && (long long)gx * gy * ((a.l1 - a.l0 + a.kpb - 1) / a.kpb) < 2LL * pcf::num_sms()) a.kpb /= 2;
     const dim3 grid((unsigned)gx, (unsigned)gy, (unsigned)((a.l1 - a.l0 + a.kpb - 1) / a.kpb));
     pcf::k_assemble<<<grid, dim3(pcf::AX, pcf::AY), pcf::ASM_SMEM, h->stream>>>(a);
     PCF_CUDA_TRY(cudaGetLastError());

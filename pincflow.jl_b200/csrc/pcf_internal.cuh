@@ -140,6 +140,17 @@ struct ReduceCtx {
     int op;
 };
 
+// SMs of the current device (148 on a B200), asked for once.
+inline int num_sms() {
+    static const int sms = [] {
+        int dev = 0, v = 0;
+        cudaGetDevice(&dev);
+        cudaDeviceGetAttribute(&v, cudaDevAttrMultiProcessorCount, dev);
+        return v > 0 ? v : 148;
+    }();
+    return sms;
+}
+
 struct Dims {
     int nx, ny, nz;
     long long n;    // nx*ny*nz

@@ -114,17 +114,6 @@ static void prof_flush(pcf_handle *h, int keep_below) {
 
 // ------------------------------------------------------------ launchers --
 
-static int num_sms() {
-    static int sms = 0;
-    if (sms == 0) {
-        int dev = 0;
-        cudaGetDevice(&dev);
-        cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-        if (sms <= 0) sms = 148;
-    }
-    return sms;
-}
-
 static ReduceCtx red(pcf_handle *h, KrylovScalars *scal, int op, double *out = nullptr) {
     ReduceCtx c;
     c.partials = h->partials;
