@@ -570,7 +570,7 @@ def run_c1(args, rank, world, local_rank):
         "metric": "time for the 200 pressure solves of 100 steps to FP64 true rel. residual 1e-10, 1 B200",
         "value": ms / 1e3, "unit": "s", "n_gpus": world, "steps": args.steps, "warmup": args.warmup,
         "ms_per_step": ms, "higher_is_better": False, "scaling": "weak", "vs_baseline": None,
-        "dtype": "f64 (grids of at most 2048 cells take the single-block FP64 solver)", "data": "synthetic",
+        "dtype": "f64 (grids of at most 2048 cells take the single-launch FP64 solver)", "data": "synthetic",
         "config": {"workload": f"c1: {WORKLOADS['c1']}", "method": METHODS[args.method],
                    "l2": "1600-cell grid: L2-resident by design (latency-bound workload)",
                    "parallelism": f"replicas x{world}"},

@@ -129,7 +129,9 @@ typedef struct {
     double inner_tolerance;        /* mixed: FP64 reliable update each time the FP32 residual fell by this factor (1e-2) */
     int max_refinements;           /* mixed: cap on restarts of the FP32 iteration after a breakdown (5) */
     int learned;                   /* mixed, bit set: 1 learned warm start, 2 learned preconditioner stage (0) */
-    int check_interval;            /* iterations per graph batch between host checks of the status word (4) */
+    int check_interval;            /* iterations per graph batch between host checks of the status word (4);
+                                      spectral solves (see multigrid) test on the device after every iteration
+                                      and do not read it */
     int restart_interval;          /* mixed: restart the Krylov recurrences at every n-th reliable update (1; 0: never) */
     int multigrid;                 /* mixed: 0: the reference preconditioner; 1: horizontal aggregation multigrid
                                       V-cycle with the reference line relaxation as smoother on every level (0).
@@ -147,7 +149,9 @@ typedef struct {
     int mg_coarse_iterations;      /* multigrid: smoothing steps on the coarsest level (4) */
     int mg_min_columns;            /* multigrid: a level with at most this many columns is the coarsest (16) */
     int autotune;                  /* 1: time the stencil tile shapes of every new grid size on first use and keep
-                                      the fastest (process-wide table, pcf_autotune_entries); 0: fixed heuristic (0) */
+                                      the fastest (process-wide table, pcf_autotune_entries); 0: fixed heuristic (0).
+                                      Spectral solves launch these stencils only where they fall back to the
+                                      V-cycle or the halos are uneven, but tune them like the others */
     int mg_operator_bf16;          /* multigrid: 1: the V-cycle's residual and smoothing stencils on the finest and
                                       the first coarse level read BF16 copies of their operators (half their bytes;
                                       the Krylov operator, the coarser levels and the FP64 true residual are
@@ -160,7 +164,8 @@ typedef struct {
                                       between the steps (column solves by warp scans).  1: on; 0: one kernel per
                                       step as on the finer levels; -1 (default): on in pcf_ensemble_solve_device
                                       (whose members' launches then leave the other SMs to one another), off in
-                                      single solves (measured slower there) */
+                                      single solves (measured slower there).  Read where the V-cycle runs; it
+                                      does not ask for the V-cycle itself (see multigrid) */
     int mg_smoother_fp8;           /* multigrid with mg_operator_bf16: the finest level's pseudo-time steps read
                                       an FP8 E4M3 copy of their 22 planes (each plane scaled by a power of 2 so
                                       that its largest value lands in [64, 128)), a quarter of the FP32 planes'
@@ -385,10 +390,12 @@ int pcf_autotune_clear(void);
  * sizes may differ.  pcf_ensemble_solve_device runs solve_poisson! for every
  * member (arrays of per-member device pointers and scalars, as
  * pcf_solve_device) with the mixed-precision iteration only: after each
- * member's setup on its own stream, every batch of check_interval
- * iterations of all members is one CUDA graph launch.  res has one entry
- * per member.  A handle may belong to one ensemble at a time and must not be
- * used by another thread while the ensemble solves. */
+ * member's setup on its own stream, the iterations of all members are one
+ * CUDA graph launch, which repeats batches of check_interval iterations (one
+ * where the members run the spectral preconditioner) until every member has
+ * finished.  res has one entry per member.  A handle may belong to one
+ * ensemble at a time and must not be used by another thread while the
+ * ensemble solves. */
 typedef struct pcf_ensemble pcf_ensemble;
 int pcf_ensemble_create(pcf_ensemble **e, pcf_handle *const *members, int count);
 int pcf_ensemble_destroy(pcf_ensemble *e);

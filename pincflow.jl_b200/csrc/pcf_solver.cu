@@ -550,10 +550,14 @@ static int apply_total(pcf_handle *h, const StencilArgs<T> &a, bool diff) {
 }
 
 // Grids of at most this many columns take the split sweep (k_thomas_split),
-// larger ones the column-per-thread sweep, which fills the GPU by itself there
-// (192x192x96 in FP32: 34 us, split 63 us).  Solves with the reference
-// preconditioner, column per thread -> split: 96x96x48 in FP64 30.2 -> 22.6 ms
-// (a sweep about 20 -> 8 us), 128x96x48 mixed 32.2 -> 27.2 ms.
+// larger ones the column-per-thread sweep, which has enough threads there
+// by itself.  us per sweep, column per thread -> split, in FP64 and FP32:
+// 64x64x32 11.3 -> 9.3, 10.9 -> 9.3; 96x96x48 18.2 -> 11.1, 16.0 -> 11.8;
+// 128x128x64 23.5 -> 18.8, 22.7 -> 15.3; 160x128x64 24.6 -> 24.1, 23.2 -> 20.7;
+// 192x192x96 40.7 -> 55.3, 33.4 -> 36.5.  Iterations with the reference
+// preconditioner: 96x96x48 in FP64 168 -> 139 us, 128x96x48 mixed 159 -> 137.
+// Both forms are equally far from exact columns (8e-17 to 2e-16 in FP64, 4e-8 to
+// 1e-7 in FP32); solves at 1e-10 end 2e-9 to 4e-8 from exact either way.
 constexpr int kSplitThomasColumns = 16384;
 
 template <typename T, int MODE>
@@ -1371,7 +1375,8 @@ static int spectral_create(pcf_handle *h) {
     s->smy = 2 * sizeof(float2) * (size_t)fpad_size(ly * ny);
     // levels per run: 4 where the columns are short (all of them in flight at
     // once), 8 from there, so that a block's chain over the runs stays short and
-    // two blocks fit an SM (256x256x128: 44 us with 4, 27 with 8), 16 beyond 256
+    // two blocks fit an SM (256x256x128: 44 us with 4, 27 with 8; 25 since one
+    // warp chains the runs), 16 beyond 256
     s->ch = nz <= 32 ? 4 : nz <= 256 ? 8 : 16;
     s->gz = dim3((unsigned)((a.npair + 31) / 32), (unsigned)ny);
     s->bz = dim3(32, (unsigned)((nz + s->ch - 1) / s->ch));
@@ -3586,12 +3591,12 @@ int pcf_profile_read(const pcf_handle *h, int tag, double *ms, long long *count,
 // ============================================================== ensemble ==
 // Mixed-precision solves of several handles (ensemble members, possibly of
 // different grid sizes) advanced together: each member's setup runs on its
-// own stream, then every batch of check_interval iterations of all members
-// is ONE CUDA graph launch (captured once per ensemble and configuration:
-// the members' iteration chains are parallel branches forked from and joined
-// to the ensemble's stream), and one status read-back per batch serves all
-// members.  Members that converge early keep returning at once from their
-// kernels (device-side done flag) until the last one finishes.
+// own stream, then the iterations of all members are ONE CUDA graph launch
+// (captured once per ensemble and configuration: a WHILE node whose body is a
+// batch of check_interval iterations, one with the spectral preconditioner; the
+// members' iteration chains are parallel branches forked from and joined to the
+// ensemble's stream).  Members that converge early keep returning at once from
+// their kernels (device-side done flag) until the last one finishes.
 
 struct pcf_ensemble {
     std::vector<pcf_handle *> m;

@@ -17,13 +17,15 @@
 // One application is five launches: x transforms (the p or s update of the
 // iteration formed on the way in), y transforms, column solves, y transforms
 // back, x transforms back.  Each moves 8-20 bytes per cell, 52 in all (the
-// V-cycle: about 330 and 60 launches).  Whole solves, V-cycle -> spectral:
-// 64x64x32 3.95 -> 0.97 ms, 150x90x45 24.2 -> 1.46 (the V-cycle's coarsening
-// ends at 75x45), 128x128x64 9.29 -> 1.87, 256x256x128 30.0 -> 7.07,
-// 512x512x192 153 -> 37.4, 32 ensemble members 186 -> 65 (with the
-// coefficient planes; in flux form, pcf_flux.cuh, less again).
-// At 512x512x192 the passes take 150-200 us where their traffic takes 62-154:
-// index arithmetic, shared-memory passes and barriers.
+// V-cycle: about 330 and 60 launches).  Whole solves, V-cycle -> spectral (with
+// the device-side loop and the flux form, pcf_flux.cuh): 64x64x32 3.97 -> 0.60
+// ms, 150x90x45 25.3 -> 1.03 (the V-cycle's coarsening ends at 75x45),
+// 128x128x64 9.33 -> 1.25, 256x256x128 30.0 -> 5.01, 512x512x192 158 -> 28.0,
+// 32 ensemble members 185 -> 37.
+// At 512x512x192 (cold, one by one): x transforms 186 us with the p update, 176
+// with the s update, y 188 either way, column solves 174, x back 152, where
+// their traffic takes 154, 123, 62, 69 and 62: index arithmetic, shared-memory
+// passes and barriers.
 //
 // Layout of the transformed field (spec): rows of nxs floats, one per (j, k),
 // holding npair complex values.  Pair i >= 1 of row j is the coefficient of

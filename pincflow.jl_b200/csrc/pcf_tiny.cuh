@@ -17,7 +17,8 @@
 // chains of 2 nz dependent FP64 steps, then the barriers.
 // One CTA with the coefficients read from L2 took 40 us per iteration on the
 // periodic hill (25 L2 loads per cell and apply, column sweeps waiting for
-// shared memory at every level); this kernel takes 24, a solve 3.29 -> 2.13 ms.
+// shared memory at every level); this kernel takes 24, a solve 3.29 -> 2.13 ms
+// (1.94 with the assembly's shorter blocks).
 //
 // Global sums run in the order of one 512-thread block (kTinySumThreads
 // partial sums over cells t, t + 512, ..., a shuffle tree per warp, then one

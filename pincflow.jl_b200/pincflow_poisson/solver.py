@@ -49,14 +49,15 @@ class PoissonNamelist:
     learned: int = 0                  # mixed, bit set: 1 learned warm start, 2 learned preconditioner stage
     check_interval: int = 4
     restart_interval: int = 1         # mixed: Krylov restart at every n-th reliable update (0: never)
-    multigrid: bool = False           # mixed: horizontal aggregation multigrid V-cycle as the preconditioner
+    multigrid: bool = False           # mixed: horizontal aggregation multigrid V-cycle as the preconditioner, or, with
+    #                                   the default settings below, the spectral inverse of the averaged operator
     mg_dtau: float = 2.5              # multigrid: pseudo-time step of the smoother on every level
     mg_coarse_iterations: int = 4     # multigrid: smoothing steps on the coarsest level
     mg_min_columns: int = 16          # multigrid: a level with at most this many columns is the coarsest
     autotune: bool = False            # time the stencil tile shapes of each new grid size on first use
     mg_operator_bf16: bool = True     # multigrid: finest and first coarse level stencils read BF16 copies
     mg_fused_coarse: Optional[bool] = None  # multigrid: levels of <= 1024 columns as one cluster launch per cycle
-    #                                         (None: in ensembles only)
+    #                                         (None: in ensembles only; read where the V-cycle runs)
     mg_smoother_fp8: bool = False     # multigrid: finest level's pseudo-time steps read an FP8 copy of their planes
 
     def to_c(self) -> _lib.PcfParams:
