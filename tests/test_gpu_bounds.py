@@ -4,8 +4,8 @@ The library built with -DPCF_BOUNDS_CHECK (build.py --checked) checks the
 global indices of its stencil, Thomas, multigrid transfer, assembly,
 corrector, spectral and flux-form kernels against their arrays' extents; an access out of range is
 skipped and recorded, never a fault.  This test runs the operator, solver,
-multigrid, corrector, predictor and spectral parity suites (small grids:
-40x1x40 up to 512x10x192, odd sizes, partial tiles) in a child process that loads that
+multigrid, corrector, predictor, spectral and column-split parity suites
+(small grids: 16x16x8 up to 512x10x192, odd sizes, partial tiles) in a child process that loads that
 library (PCF_LIB_VARIANT=checked); there every test also asserts that no
 access was out of range (tests/conftest.py), on top of its elementwise
 comparison with the oracle.
@@ -20,7 +20,7 @@ pytestmark = pytest.mark.gpu
 
 HERE = os.path.dirname(os.path.abspath(__file__))
 SUITES = ["test_gpu_parity.py", "test_gpu_multigrid.py", "test_gpu_corrector.py", "test_gpu_predictor.py",
-          "test_gpu_lhs.py", "test_gpu_spectral.py"]
+          "test_gpu_lhs.py", "test_gpu_spectral.py", "test_gpu_column_splits.py"]
 
 
 def test_parity_suites_on_the_bounds_checked_build():

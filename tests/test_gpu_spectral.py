@@ -195,3 +195,40 @@ def test_flux_form_of_a_constant_is_zero(name, pcf):
             pi = np.full(cfg["dom"].interior_shape, value)
             for precision in ("fp64", "fp32"):
                 assert not s.apply_flux(pi, precision).any(), (value, precision)
+
+
+@pytest.mark.parametrize("name", ["rho", "comp", "200x1x40", "1x100x30"])
+def test_solve_in_flux_form(name, pcf):
+    """Solves that end in the flux form: density, damping and the Compressible
+    model with even halos, and grids of one row along x or y."""
+    if "x" in name:
+        nx, ny, nz = (int(v) for v in name.split("x"))
+        cfg = dict(C.c3(31, nx=nx, ny=ny, nz=nz), damp=False, p=None)
+    else:
+        cfg = dict(case(name))
+    dom = cfg["dom"]
+    for key in ("rho", "betar", "p"):
+        if cfg[key] is not None:
+            cfg[key] = _periodic(dom, cfg[key])
+    with pcf.PoissonSolver(dom, cfg["model"]) as s:
+        s.set_grid(cfg["fields"])
+        s.set_background(cfg["fields"])
+        s.compute_operator(cfg["rho"], cfg["betar"], cfg["dt"], cfg["rayleigh_factor"], cfg["damp"], cfg["p"],
+                           return_coef=False)
+        want = np.random.default_rng(9).standard_normal(dom.interior_shape)
+        rhs = s.apply_operator(want)
+        dpip = np.zeros(dom.halo_shape)
+        info = s.solve_poisson(rhs, cfg["rho"], cfg["betar"], cfg["dt"], cfg["rayleigh_factor"], 1.0,
+                               pcf.PoissonNamelist(tolerance=1e-10, tolerance_is_relative=True, precision="mixed",
+                                                   multigrid=True, damp_horizontal_wind_on_rhs=cfg["damp"]),
+                               dpip, p=cfg["p"])
+        assert not info.errflag and info.niter <= 12, info
+        fc = F.fcscal(dom, cfg["fields"])
+        x = dom.interior(dpip) * fc * cfg["dt"]
+        s.apply_flux(x / fc)  # (an error if the solve went on with the planes)
+        r = rhs - s.apply_operator(x)
+        assert np.sqrt((r ** 2).mean() / (rhs ** 2).mean()) <= 1.01e-10
+    got, want = x / fc, want / fc
+    if cfg["model"] != "Compressible":  # the pressure's free constant
+        got, want = got - got.mean(), want - want.mean()
+    assert rel_err(got, want) < 1e-6
