@@ -1,12 +1,12 @@
 """GPU: the parity suites on the bounds-checked build.
 
 The library built with -DPCF_BOUNDS_CHECK (build.py --checked) checks the
-global indices of its stencil, Thomas, multigrid transfer, assembly,
-corrector, spectral and flux-form kernels against their arrays' extents; an access out of range is
-skipped and recorded, never a fault.  This test runs the operator, solver,
-multigrid, corrector, predictor, spectral and column-split parity suites
-(small grids: 16x16x8 up to 512x10x192, odd sizes, partial tiles) in a child process that loads that
-library (PCF_LIB_VARIANT=checked); there every test also asserts that no
+global indices of its stencil, Thomas, multigrid transfer, assembly, corrector,
+spectral and flux-form kernels against their arrays' extents; an access out of
+range is skipped and recorded, never a fault.  This test runs the operator,
+solver, multigrid, corrector, predictor, spectral and column-split parity
+suites (small grids: 16x16x8 up to 512x10x192, odd sizes, partial tiles) in a
+child process that loads that library (PCF_LIB_VARIANT=checked); there every test also asserts that no
 access was out of range (tests/conftest.py), on top of its elementwise
 comparison with the oracle.
 """
